@@ -38,15 +38,24 @@
 #define FPM_COL_MINB_1024 1
 #endif
 #ifndef FPM_COL_MINB_512
-#define FPM_COL_MINB_512 1
+#define FPM_COL_MINB_512 2
 #endif
 template <int N> struct ColTZ {
     static constexpr int v = N == 1024 ? FPM_COL_TZ_1024
                            : N == 512 ? FPM_COL_TZ_512
                            : (ColPlan<N>::T >= 32 ? 8 : 16);
 };
+// CTAs per SM the column kernels are compiled for: with every load of a line
+// issued up front the passes want bytes in flight, so the 8-element plans
+// (64 registers) run 4 CTAs of 128-256 threads (y pass at n = 256: 39.7 us with
+// 2, 35 with 3, 31 with 4), n = 512 two of 512 threads (379 -> 260 us), n = 192
+// three (23 -> 18.8 us); the 24-element plans of the other 3 2^k lines two
 template <int N> struct ColMinB {
-    static constexpr int v = N == 1024 ? FPM_COL_MINB_1024 : N == 512 ? FPM_COL_MINB_512 : 2;
+    static constexpr int v = N == 1024 ? FPM_COL_MINB_1024
+                           : N == 512 ? FPM_COL_MINB_512
+                           : N == 192 ? 3
+                           : N % 3 == 0 ? 2
+                                        : 4;
 };
 constexpr int pow2_factor(long long x) {
     int p = 1;
@@ -261,24 +270,34 @@ FPM_DEV void col_tile(const PassArgs& a, int zt, int o_idx, float2* smem, int sl
         const OutSpec os = a.o[o];
         const float2* src = a.in[os.src] + slot * a.in_ss[os.src];
         float2* dst = (float2*)a.out[o] + slot * a.out_ss[o];
+        // every load of the line first, the transfer on the registers after
+        // them: with its branches between the loads they went out one at a time
         auto LD = [&](int pos) -> float2 {
-            float2 x;
-            if (FWD) x = held[pos * TZ + c];
-            else if (SRC_SM) x = tin[pos * TZ + c];
-            else x = valid ? ldg2<CG>(src + base + pos * estride) : make_float2(0.f, 0.f);
-            float coef = os.coef;
-            if (AXIS == 0 && a.laplace) {
-                const int nx = signed_n<N>(pos);
-                const int n2 = n2t + nx * nx;
-                coef = n2 == 0 ? 0.f : coef * lap_over(lapcoef, n2) * shell_at(a.shell, n2);
-            }
-            const float ga = os.pw ? grad_a<N>(pos, a.inv6h) : 0.f;
-            return apply_pw(x, os.pw, ga, coef);
+            if (FWD) return held[pos * TZ + c];
+            if (SRC_SM) return tin[pos * TZ + c];
+            return valid ? ldg2<CG>(src + base + pos * estride) : make_float2(0.f, 0.f);
         };
         auto ST = [&](int pos, float2 x) {
             if (valid) dst[base + pos * estride] = x;
         };
         LI::load(v, t, LD);
+        const bool lap = AXIS == 0 && a.laplace;
+        if (lap || os.pw || os.coef != 1.f) {   // block-uniform
+            constexpr int T = PL::T, R0 = RadixEnds<typename PL::R>::first;
+#pragma unroll
+            for (int k = 0; k < E; ++k) {
+                const int pos = t + T * k;
+                float2& x = v[(k % (E / R0)) * R0 + k / (E / R0)];
+                float coef = os.coef;
+                if (lap) {
+                    const int nx = signed_n<N>(pos);
+                    const int n2 = n2t + nx * nx;
+                    coef = n2 == 0 ? 0.f : coef * lap_over(lapcoef, n2) * shell_at(a.shell, n2);
+                }
+                const float ga = os.pw ? grad_a<N>(pos, a.inv6h) : 0.f;
+                x = apply_pw(x, os.pw, ga, coef);
+            }
+        }
         if (SRC_SM && !FWD && TWOA && a.nout == 1) {
             // one output: the loaded tile is free once in registers, so the
             // exchanges alternate between the work area and the tile
