@@ -46,16 +46,12 @@ template <int N> struct ColTZ {
                            : (ColPlan<N>::T >= 32 ? 8 : 16);
 };
 // CTAs per SM the column kernels are compiled for: with every load of a line
-// issued up front the passes want bytes in flight, so the 8-element plans
-// (64 registers) run 4 CTAs of 128-256 threads (y pass at n = 256: 39.7 us with
-// 2, 35 with 3, 31 with 4), n = 512 two of 512 threads (379 -> 260 us), n = 192
-// three (23 -> 18.8 us); the 24-element plans of the other 3 2^k lines two
+// issued up front the passes want bytes in flight, so the 8- and 12-element
+// plans (64 registers) run 4 CTAs of 128-256 threads (y pass at n = 256: 39.7 us
+// with 2, 35 with 3, 31 with 4; n = 384: 150 / 127 / 119 us), n = 512 two of 512
+// threads (379 -> 260 us)
 template <int N> struct ColMinB {
-    static constexpr int v = N == 1024 ? FPM_COL_MINB_1024
-                           : N == 512 ? FPM_COL_MINB_512
-                           : N == 192 ? 3
-                           : N % 3 == 0 ? 2
-                                        : 4;
+    static constexpr int v = N == 1024 ? FPM_COL_MINB_1024 : N == 512 ? FPM_COL_MINB_512 : 4;
 };
 constexpr int pow2_factor(long long x) {
     int p = 1;
@@ -657,8 +653,11 @@ FPM_DEV void r2c_rows(const float* __restrict__ real, float2* __restrict__ cplx,
 #ifndef FPM_C2R_MINB
 #define FPM_C2R_MINB 3
 #endif
+// 4 for the 12-element rows of n = 3 2^k (64 registers; n = 384 c2r 126 us with
+// 2, 107 with 3, 103 with 4)
 template <int N, int B> struct RowMinB {
-    static constexpr int v = Plan<N / 2>::T * RowTR<N / 2>::v * B <= 2048 ? B : 1;
+    static constexpr int w = N % 3 == 0 ? 4 : B;
+    static constexpr int v = Plan<N / 2>::T * RowTR<N / 2>::v * w <= 2048 ? w : 1;
 };
 
 template <int N>
@@ -737,6 +736,44 @@ FPM_DEV void discard_row(const float2* row, int zp, int t, int T) {
         asm volatile("discard.global.L2 [%0], 128;" ::"l"(p + q * 128) : "memory");
 }
 
+// Thread t loads X_k for k = t + T q (q < E), lane 0 also X_M; the
+// partner X_{M-k} of k = t + T q sits in lane T - t of the row's
+// T-lane group at q' = E - 1 - q (lane 0: its own E - q, or X_M for
+// q = 0), so Z_k is formed with shuffles, without a shared row,
+// straight into the first stage's registers (element t + T q is
+// v[(q % E0) R0 + q / E0], R0 the first radix, E0 = E / R0).
+template <int M, bool CG>
+FPM_DEV void c2r_load_shfl(const float2* in, int pw, float coef, float inv6h, int t, float2* v) {
+    constexpr int N = 2 * M, T = Plan<M>::T, E = Plan<M>::E;
+    constexpr int R0 = RadixEnds<typename Plan<M>::R>::first, E0 = E / R0;
+    float2 xv[E];
+#pragma unroll
+    for (int q = 0; q < E; ++q) xv[q] = ldg2<CG>(in + t + T * q);
+    float2 xM = t == 0 ? ldg2<CG>(in + M) : make_float2(0.f, 0.f);
+#pragma unroll
+    for (int q = 0; q < E; ++q) {
+        const int k = t + T * q;
+        float2 x = xv[q];
+        if (k == 0) x.y = 0.f;   // Hermitian: imaginary parts of DC / Nyquist unused
+        xv[q] = apply_pw(x, pw, pw ? grad_a<N>(k, inv6h) : 0.f, coef);
+    }
+    xM.y = 0.f;
+    xM = apply_pw(xM, pw, pw ? grad_a<N>(M, inv6h) : 0.f, coef);
+    const int partner = (T - t) % T;
+#pragma unroll
+    for (int q = 0; q < E; ++q) {
+        const float2 bq = xv[E - 1 - q];
+        float2 xm = make_float2(__shfl_sync(0xffffffffu, bq.x, partner, T),
+                                __shfl_sync(0xffffffffu, bq.y, partner, T));
+        if (t == 0) xm = q == 0 ? xM : xv[(E - q) % E];
+        xm = c_conj(xm);
+        const float2 xk = xv[q];
+        const float2 s2 = c_add(xk, xm);
+        const float2 w = c_mul(twiddle<N, +1>(t + T * q), c_sub(xk, xm));
+        v[(q % E0) * R0 + q / E0] = make_float2(s2.x - w.y, s2.y + w.x);
+    }
+}
+
 // TR rows starting at row0; outputs stored with evict-first hints when the
 // rows are produced inside a fused kernel (STREAM), inputs dropped from L2
 // after use when DISCARD.
@@ -755,39 +792,7 @@ FPM_DEV void c2r_rows(const PassArgs& a, long long row0, float2* smem, int slot 
             auto LD = [&](int pos) -> float2 { return c2r_pre_direct<M, CG>(in, pos, os.pw, os.coef, a.inv6h); };
             WLine<M, +1>::load(v, t, LD);
         } else if (WarpLocal<M>::v && FPM_C2R_SHFL) {
-            // Thread t loads X_k for k = t + T q (q < E), lane 0 also X_M; the
-            // partner X_{M-k} of k = t + T q sits in lane T - t of the row's
-            // T-lane group at q' = E - 1 - q (lane 0: its own E - q, or X_M for
-            // q = 0), so Z_k is formed with shuffles, without a shared row,
-            // straight into the first stage's registers (element t + T q is
-            // v[(q % E0) R0 + q / E0], R0 the first radix, E0 = E / R0).
-            constexpr int R0 = RadixEnds<typename Plan<M>::R>::first, E0 = E / R0;
-            float2 xv[E];
-#pragma unroll
-            for (int q = 0; q < E; ++q) xv[q] = ldg2<CG>(in + t + T * q);
-            float2 xM = t == 0 ? ldg2<CG>(in + M) : make_float2(0.f, 0.f);
-#pragma unroll
-            for (int q = 0; q < E; ++q) {
-                const int k = t + T * q;
-                float2 x = xv[q];
-                if (k == 0) x.y = 0.f;   // Hermitian: imaginary parts of DC / Nyquist unused
-                xv[q] = apply_pw(x, os.pw, os.pw ? grad_a<N>(k, a.inv6h) : 0.f, os.coef);
-            }
-            xM.y = 0.f;
-            xM = apply_pw(xM, os.pw, os.pw ? grad_a<N>(M, a.inv6h) : 0.f, os.coef);
-            const int partner = (T - t) % T;
-#pragma unroll
-            for (int q = 0; q < E; ++q) {
-                const float2 bq = xv[E - 1 - q];
-                float2 xm = make_float2(__shfl_sync(0xffffffffu, bq.x, partner, T),
-                                        __shfl_sync(0xffffffffu, bq.y, partner, T));
-                if (t == 0) xm = q == 0 ? xM : xv[(E - q) % E];
-                xm = c_conj(xm);
-                const float2 xk = xv[q];
-                const float2 s2 = c_add(xk, xm);
-                const float2 w = c_mul(twiddle<N, +1>(t + T * q), c_sub(xk, xm));
-                v[(q % E0) * R0 + q / E0] = make_float2(s2.x - w.y, s2.y + w.x);
-            }
+            c2r_load_shfl<M, CG>(in, os.pw, os.coef, a.inv6h, t, v);
         } else {
             c2r_load_row<M, CG>(S, in, os.pw, os.coef, a.inv6h, t);
             stage_sync<WarpLocal<M>::v>();
@@ -1250,32 +1255,37 @@ fused_y_inv_z_c2r(PassArgs y, PassArgs z, int pb, int lag, QueueCtl* q) {
 // z pass for the 2LPT source: six c2r rows combined in registers into
 //   scale * [phi_xx phi_yy + phi_yy phi_zz + phi_zz phi_xx - phi_xy^2 - phi_yz^2 - phi_zx^2]
 // outputs 0..5 must be (xx, yy, zz, xy, yz, zx).
+// A row's threads sit in one warp (WarpLocal), so the six transforms need warp
+// barriers only and pair X_k with X_{M-k} by shuffles, as c2r_rows does: bound
+// by its instructions and the sums it holds in registers (n = 256: 284 -> 162
+// us, n = 512: 2208 -> 1211 us; the six inputs alone take 80 / 620 us of HBM).
+// FPM_LPT2_MINB: CTAs per SM (n = 512: 1395 us with 1, 1211 with 2, 1394 with 3).
+#ifndef FPM_LPT2_MINB
+#define FPM_LPT2_MINB 2
+#endif
 template <int N>
-__global__ void __launch_bounds__(Plan<N / 2>::T * RowTR<N / 2>::v)
+__global__ void __launch_bounds__(Plan<N / 2>::T * RowTR<N / 2>::v, FPM_LPT2_MINB)
 row_c2r_lpt2(PassArgs a) {
     constexpr int M = N / 2, T = Plan<M>::T, E = Plan<M>::E, TR = RowTR<M>::v;
+    static_assert(WarpLocal<M>::v, "a row's threads share a warp");
     extern __shared__ float2 smem[];
     const int r = threadIdx.x / T, t = threadIdx.x % T;
     const long long row = (long long)blockIdx.x * TR + r;
     const PadRow S{smem + r * RowSm<M>::v};
     auto SM = [&](int pos) -> float2& { return S[pos]; };
     float2 v[E], sum[E], acc[E];
+    float2* out = reinterpret_cast<float2*>((float*)a.out[0] + row * N);
+    const float sc = a.scale;
+#pragma unroll
     for (int o = 0; o < 6; ++o) {
         const OutSpec os = a.o[o];
-        c2r_load_row<M, false>(S, a.in[os.src] + row * a.zp, os.pw, os.coef, a.inv6h, t);
-        __syncthreads();
-        auto LD = [&](int pos) -> float2 { return c2r_pre<M>(S, pos); };
-        Line<M, +1>::load(v, t, LD);
-        __syncthreads();
+        c2r_load_shfl<M, false>(a.in[os.src] + row * a.zp, os.pw, os.coef, a.inv6h, t, v);
         // the last stage hands each thread the same positions for every output,
         // in the same order, so a running slot counter indexes sum/acc.
         int slot = 0;
-        float2* out = reinterpret_cast<float2*>((float*)a.out[0] + row * N);
-        const float sc = a.scale;
         auto ST = [&](int pos, float2 x) {
             if (o == 0) {
                 sum[slot] = x;
-                acc[slot] = make_float2(0.f, 0.f);
             } else if (o == 1) {
                 acc[slot] = make_float2(sum[slot].x * x.x, sum[slot].y * x.y);
                 sum[slot] = c_add(sum[slot], x);
@@ -1289,8 +1299,8 @@ row_c2r_lpt2(PassArgs a) {
             }
             ++slot;
         };
-        Line<M, +1>::run(v, t, SM, ST);
-        __syncthreads();
+        WLine<M, +1>::run(v, t, SM, ST);
+        stage_sync<WarpLocal<M>::v>();
     }
 }
 

@@ -78,6 +78,58 @@ template <int DIR> struct DFT<4, DIR> {
     FPM_DEV static void run(float2* v) { dft4<DIR>(v[0], v[1], v[2], v[3]); }
 };
 
+template <int DIR> struct DFT<6, DIR> {
+    // n = 3 n1 + n2 (n1 < 2, n2 < 3), k = k1 + 2 k2: three 2-point DFTs over
+    // n1, twiddles W6^{n2 k1}, two 3-point DFTs over n2
+    FPM_DEV static void run(float2* v) {
+        float2 e[3], o[3];
+#pragma unroll
+        for (int n2 = 0; n2 < 3; ++n2) {
+            e[n2] = c_add(v[n2], v[n2 + 3]);
+            o[n2] = c_sub(v[n2], v[n2 + 3]);
+        }
+        // W6 = 1/2 + DIR i sqrt(3)/2, W6^2 = -1/2 + DIR i sqrt(3)/2
+        o[1] = make_float2(0.5f * o[1].x - DIR * FPM_SQRT3_2 * o[1].y, 0.5f * o[1].y + DIR * FPM_SQRT3_2 * o[1].x);
+        o[2] = make_float2(-0.5f * o[2].x - DIR * FPM_SQRT3_2 * o[2].y, -0.5f * o[2].y + DIR * FPM_SQRT3_2 * o[2].x);
+        DFT<3, DIR>::run(e);
+        DFT<3, DIR>::run(o);
+#pragma unroll
+        for (int k2 = 0; k2 < 3; ++k2) {
+            v[2 * k2] = e[k2];
+            v[2 * k2 + 1] = o[k2];
+        }
+    }
+};
+
+template <int DIR> struct DFT<12, DIR> {
+    // n = 3 n1 + n2 (n1 < 4, n2 < 3), k = k1 + 4 k2: three 4-point DFTs over
+    // n1, twiddles W12^{n2 k1}, four 3-point DFTs over n2
+    FPM_DEV static void run(float2* v) {
+        float2 y[3][4];
+#pragma unroll
+        for (int n2 = 0; n2 < 3; ++n2) {
+#pragma unroll
+            for (int n1 = 0; n1 < 4; ++n1) y[n2][n1] = v[3 * n1 + n2];
+            dft4<DIR>(y[n2][0], y[n2][1], y[n2][2], y[n2][3]);
+        }
+        constexpr float C = FPM_SQRT3_2, S = 0.5f * DIR;   // W12 = C + i S
+        y[1][1] = make_float2(C * y[1][1].x - S * y[1][1].y, C * y[1][1].y + S * y[1][1].x);               // W12
+        y[1][2] = make_float2(0.5f * y[1][2].x - DIR * C * y[1][2].y, 0.5f * y[1][2].y + DIR * C * y[1][2].x);   // W12^2
+        y[1][3] = c_muli<DIR>(y[1][3]);                                                                       // W12^3
+        y[2][1] = make_float2(0.5f * y[2][1].x - DIR * C * y[2][1].y, 0.5f * y[2][1].y + DIR * C * y[2][1].x);   // W12^2
+        y[2][2] = make_float2(-0.5f * y[2][2].x - DIR * C * y[2][2].y, -0.5f * y[2][2].y + DIR * C * y[2][2].x); // W12^4
+        y[2][3] = make_float2(-y[2][3].x, -y[2][3].y);                                                        // W12^6
+#pragma unroll
+        for (int k1 = 0; k1 < 4; ++k1) {
+            float2 t[3] = {y[0][k1], y[1][k1], y[2][k1]};
+            DFT<3, DIR>::run(t);
+            v[k1] = t[0];
+            v[k1 + 4] = t[1];
+            v[k1 + 8] = t[2];
+        }
+    }
+};
+
 template <int DIR> struct DFT<8, DIR> {
     FPM_DEV static void run(float2* v) {
         float2 e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6];
@@ -208,6 +260,11 @@ template <int R0, int... Rs> struct RadixEnds<Radices<R0, Rs...>> {
     static constexpr int last = all[sizeof...(Rs)];
 };
 
+// Lines of 24 to 384 points with a factor 3 take 12 elements per thread (radix
+// 12 or 6 first): with 24 (radix 3 first) the row passes spilled at the
+// occupancy they want and the column passes ran at half of it (n = 384: r2c 131
+// -> 104 us, c2r 154 -> 103, x forward + inverse 206 -> 181, 2LPT source rows
+// 1255 -> 618).
 template <int N> struct Plan;
 #define FPM_PLAN(N_, T_, ...)                                  \
     template <> struct Plan<N_> {                              \
@@ -217,15 +274,15 @@ template <int N> struct Plan;
 FPM_PLAN(8, 1, 8)
 FPM_PLAN(12, 1, 3, 4)
 FPM_PLAN(16, 1, 16)
-FPM_PLAN(24, 1, 3, 8)
+FPM_PLAN(24, 2, 6, 4)
 FPM_PLAN(32, 2, 16, 2)
-FPM_PLAN(48, 2, 3, 8, 2)
+FPM_PLAN(48, 4, 12, 4)
 FPM_PLAN(64, 4, 16, 4)
-FPM_PLAN(96, 4, 3, 8, 4)
+FPM_PLAN(96, 8, 6, 4, 4)
 FPM_PLAN(128, 8, 16, 8)
-FPM_PLAN(192, 8, 3, 8, 8)
+FPM_PLAN(192, 16, 12, 4, 4)
 FPM_PLAN(256, 16, 16, 16)
-FPM_PLAN(384, 16, 3, 8, 4, 4)
+FPM_PLAN(384, 32, 6, 4, 4, 4)
 FPM_PLAN(512, 32, 16, 8, 4)
 FPM_PLAN(1024, 64, 16, 16, 4)
 
