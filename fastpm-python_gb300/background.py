@@ -39,11 +39,14 @@ class MatterDominated(object):
         """background.py:186-205: odeint on the ln a grid, normalised to 1 at
         the grid point nearest a_normalize."""
         lna = self.lna
-        y = odeint(self.ode, y0, lna, tcrit=[0.], atol=0)
+        rhs = self.ode
+        if type(self) is MatterDominated and self.Omega0_m > 0 and self.Omega0_k >= 0 and self.Omega0_lambda >= 0:
+            rhs = self._ode_floats
+        y = odeint(rhs, y0, lna, tcrit=[0.], atol=0)
         v1 = numpy.empty((len(lna), 3))
         v2 = numpy.empty((len(lna), 3))
         for i, (yi, lnai) in enumerate(zip(y, lna)):
-            d1p, f1p, d2p, f2p = self.ode(yi, lnai)
+            d1p, f1p, d2p, f2p = rhs(yi, lnai)
             v1[i] = (yi[0], yi[1], f1p)
             v2[i] = (yi[2], yi[3], f2p)
         ind = abs(lna - numpy.log(a_normalize)).argmin()
@@ -70,6 +73,19 @@ class MatterDominated(object):
         a = numpy.exp(lna)
         hfac = self.Hfac(a)
         omega = self.Om(a)
+        return F1, hfac * F1 + 1.5 * omega * D1, F2, hfac * F2 + 1.5 * omega * D2 - 1.5 * omega * D1 ** 2
+
+    def _ode_floats(self, y, lna):
+        """ode on Python floats, Hfac and Om written out: the same operations
+        in the same order, so the same bits.  odeint calls it some 470 times a
+        solve, nearly all of which was numpy's scalar arithmetic (a solve took
+        2.1 ms, now 0.84)."""
+        D1, F1, D2, F2 = y.tolist()
+        a = float(numpy.exp(lna))
+        Om, Ok = self.Omega0_m, self.Omega0_k
+        ea = (Om / a ** 3 + Ok / a ** 2 + self.Omega0_lambda) ** 0.5
+        hfac = -2. - 0.5 / ea * (-3 * Om / (a ** 4) + -2 * Ok / (a ** 3)) * a / ea
+        omega = (Om / a ** 3) / ea ** 2
         return F1, hfac * F1 + 1.5 * omega * D1, F2, hfac * F2 + 1.5 * omega * D2 - 1.5 * omega * D1 ** 2
 
     def D1(self, a, order=0):
