@@ -12,6 +12,7 @@
 // stage) and stored once from registers (last stage); the stages in between
 // exchange through shared memory.
 #include "fft_engine.cuh"
+#include "ff.cuh"
 #include "force_readout.h"
 #include "trace.h"
 
@@ -1323,61 +1324,130 @@ FPM_DEV void philox4x32_10(uint32_t c[4], uint32_t k0, uint32_t k1) {
         c[3] = lo0;
     }
 }
-FPM_DEV double u53(uint32_t a, uint32_t b) {
-    return ((double)(a >> 5) * 67108864.0 + (double)(b >> 6) + 0.5) * (1.0 / 9007199254740992.0);
-}
-FPM_DEV void wn_draw(long long lin, uint32_t k0, uint32_t k1, double& u1, double& u2) {
-    uint32_t c[4] = {(uint32_t)(lin & 0xFFFFFFFFll), (uint32_t)(lin >> 32), 0u, 0u};
+// Mode values.  The reference numbers are float64 (Box-Muller of two 53-bit
+// uniforms), rounded to float32; in FP64 the logarithm, square root and
+// sincospi bound the kernel (256^3: 1550 us).  Here they are float-float
+// (ff.cuh), good to about 2^-38, so all but some 1e-4 of the modes round to
+// the same float32 and the error against float64 is the rounding either way.
+//   log: table-driven (Tang 1990), u = 2^e f with f inv_k = 1 + r, |r| <= 2^-7,
+//     and the series of log(1 + r); entries next to f = 1 and 2 have inv_k = 1
+//     and 1/2 exactly, so r keeps the relative accuracy of -log(u) at u -> 1.
+//   sin, cos of 2 pi u2: the nearest of 256 table angles and a short Taylor
+//     step, |theta| <= 2 pi / 512.
+// Each uniform is V / 2^54 with V the odd 54-bit integer 2 v + 1 of its 53 bits.
+static __device__ float4 g_wn_log[128];    // inv, (-log inv).h, .l, exponent step
+static __device__ float4 g_wn_trig[256];   // cos.h, cos.l, sin.h, sin.l
+
+FPM_DEV void wn_draw(unsigned long long lin, uint32_t k0, uint32_t k1, unsigned long long& v1,
+                     unsigned long long& v2) {
+    uint32_t c[4] = {(uint32_t)lin, (uint32_t)(lin >> 32), 0u, 0u};
     philox4x32_10(c, k0, k1);
-    u1 = u53(c[0], c[1]);
-    u2 = u53(c[2], c[3]);
+    v1 = ((((unsigned long long)(c[0] >> 5)) << 26 | (c[1] >> 6)) << 1) | 1ull;
+    v2 = ((((unsigned long long)(c[2] >> 5)) << 26 | (c[3] >> 6)) << 1) | 1ull;
+}
+// a non-negative integer below 2^63 as float-float (its leading 48 bits)
+FPM_DEV ff ff_of_u64(unsigned long long x) {
+    const float h = __ull2float_rz(x);
+    return ff_quick(h, __ull2float_rn(x - (unsigned long long)h));
+}
+// -log(V / 2^54)
+FPM_DEV ff wn_neg_log(unsigned long long V) {
+    const int lz = __clzll((long long)V);
+    const unsigned long long m = V << lz;              // f = m / 2^63 in [1, 2)
+    const int idx = (int)((m >> 56) & 127);
+    const float4 t = __ldg(&g_wn_log[idx]);
+    float e = (float)(9 - lz) + t.w;                    // u = f 2^(9 - lz)
+    ff r;
+    if (idx == 0) {                                     // f - 1, exact
+        const ff g = ff_of_u64(m - (1ull << 63));
+        r = ff_of(g.h * 0x1p-63f, g.l * 0x1p-63f);
+    } else if (idx == 127) {                            // f / 2 - 1, exact
+        const ff g = ff_of_u64(0ull - m);               // 2^64 - m
+        r = ff_of(g.h * -0x1p-64f, g.l * -0x1p-64f);
+    } else {
+        const unsigned hi = (unsigned)(m >> 40);        // 24 leading bits, 24 more
+        const unsigned lo = (unsigned)(m >> 16) & 0xffffffu;
+        const float fh = (float)hi * 0x1p-23f, fl = (float)lo * 0x1p-47f;
+        const ff p = ff_two_prod(fh, t.x);
+        r = ff_quick(__fsub_rn(p.h, 1.f), __fmaf_rn(fl, t.x, p.l));
+    }
+    // log(1 + r) = r - r^2 / 2 + r^3 (1/3 - r/4 + r^2/5 - r^3/6)
+    const float x = r.h;
+    const float c = __fmaf_rn(x, __fmaf_rn(x, __fmaf_rn(x, -1.f / 6.f, 0.2f), -0.25f), 1.f / 3.f);
+    const ff x2 = ff_two_prod(x, x);
+    const float lo = __fmaf_rn(x2.h * x, c, __fmaf_rn(-x, r.l, -0.5f * x2.l));
+    ff s = ff_quick(x, -0.5f * x2.h);
+    s = ff_quick(s.h, __fadd_rn(s.l, __fadd_rn(r.l, lo)));
+    // + e log 2 - log inv
+    constexpr float LN2H = (float)M_LN2, LN2L = (float)(M_LN2 - (double)(float)M_LN2);
+    if (e != 0.f || t.y != 0.f) {
+        const ff el = ff_two_prod(e, LN2H);
+        s = ff_add(ff_add(ff_quick(el.h, __fmaf_rn(e, LN2L, el.l)), ff_of(t.y, t.z)), s);
+    }
+    return ff_neg(s);
+}
+// cos and sin of 2 pi V / 2^54
+FPM_DEV void wn_sincos(unsigned long long V, ff& c, ff& s) {
+    const unsigned k = (unsigned)((V + (1ull << 45)) >> 46);       // nearest of 256 angles
+    const long long d = (long long)V - ((long long)k << 46);      // |d| <= 2^45
+    const float4 t = __ldg(&g_wn_trig[k & 255u]);
+    const float dh = __ll2float_rn(d);
+    const float dl = __ll2float_rn(d - (long long)dh);
+    constexpr float TPH = (float)(2.0 * M_PI), TPL = (float)(2.0 * M_PI - (double)(float)(2.0 * M_PI));
+    const float a = dh * 0x1p-54f;
+    ff th = ff_two_prod(a, TPH);
+    th = ff_quick(th.h, __fmaf_rn(a, TPL, __fmaf_rn(dl * 0x1p-54f, TPH, th.l)));
+    const float x = th.h, x2 = x * x;
+    const float ds = x * x2 * __fmaf_rn(x2, 1.f / 120.f, -1.f / 6.f);       // sin - theta
+    const float c1 = x2 * __fmaf_rn(x2, __fmaf_rn(x2, -1.f / 720.f, 1.f / 24.f), -0.5f);   // cos - 1
+    const ff sn = ff_quick(th.h, __fadd_rn(th.l, ds));
+    // cos(A + th) = C + (C c1 - S sin th), sin(A + th) = S + (S c1 + C sin th)
+    const ff cs = ff_mul(ff_of(t.z, t.w), ff_neg(sn)), cc = ff_mul(ff_of(t.x, t.y), sn);
+    c = ff_add(ff_of(t.x, t.y), ff_add_f(cs, t.x * c1));
+    s = ff_add(ff_of(t.z, t.w), ff_add_f(cc, t.z * c1));
+}
+FPM_DEV float ff_round_mul(ff a, ff b) {
+    const ff p = ff_mul(a, b);
+    return __fadd_rn(p.h, p.l);
 }
 
-__global__ void whitenoise_kernel(float2* out, int n, int zp, uint32_t k0, uint32_t k1,
-                                  int unitary, double mean) {
+// one thread per mode, a warp along l; grid-stride over the n^2 rows
+__global__ void __launch_bounds__(256) whitenoise_kernel(float2* out, int n, int zp, uint32_t k0, uint32_t k1,
+                                                         int unitary, float mean) {
     const int nz = n / 2 + 1;
-    const long long total = (long long)n * n * nz;
-    for (long long m = blockIdx.x * (long long)blockDim.x + threadIdx.x; m < total;
-         m += (long long)gridDim.x * blockDim.x) {
-        const int l = (int)(m % nz);
-        const long long ij = m / nz;
-        const int j = (int)(ij % n), i = (int)(ij / n);
-        const bool plane = (l == 0) || (l == n / 2);
-        double re, im;
-        if (!plane) {
-            double u1, u2;
-            wn_draw(m, k0, k1, u1, u2);
-            double s, c;
-            sincospi(2.0 * u2, &s, &c);
-            const double amp = unitary ? 1.0 : sqrt(-log(u1));
-            re = amp * c;
-            im = amp * s;
-        } else {
-            const int mi = (n - i) % n, mj = (n - j) % n;
-            const long long lin2 = (long long)i * n + j, mlin2 = (long long)mi * n + mj;
-            if (lin2 == mlin2) {  // self-conjugate: real
-                double u1, u2;
-                wn_draw(m, k0, k1, u1, u2);
-                double c = cospi(2.0 * u2);
-                re = unitary ? (c >= 0 ? 1.0 : -1.0) : sqrt(-2.0 * log(u1)) * c;
-                im = 0.0;
+    const int nrow = n * n;
+    const int lane = threadIdx.x & 31;
+    for (int ij = blockIdx.x * 8 + (threadIdx.x >> 5); ij < nrow; ij += gridDim.x * 8) {
+        const int i = ij / n, j = ij - i * n;
+        const int mij = (i == 0 ? 0 : n - i) * n + (j == 0 ? 0 : n - j);   // the row of (-i, -j)
+        for (int l = lane; l < nz; l += 32) {
+            // on the l = 0 and l = n/2 planes a pair of modes takes the draw of
+            // the lower one, a self-conjugate mode is real
+            const bool plane = l == 0 || l == n / 2;
+            const bool mirror = plane && ij > mij, self = plane && ij == mij;
+            unsigned long long v1, v2;
+            wn_draw((unsigned long long)(mirror ? mij : ij) * nz + l, k0, k1, v1, v2);
+            ff c, s;
+            wn_sincos(v2, c, s);
+            float re, im;
+            if (unitary) {
+                re = self ? (c.h >= 0.f ? 1.f : -1.f) : __fadd_rn(c.h, c.l);
+                im = __fadd_rn(s.h, s.l);
             } else {
-                const bool mirror = lin2 > mlin2;
-                const long long src = mirror ? (mlin2 * nz + l) : m;
-                double u1, u2;
-                wn_draw(src, k0, k1, u1, u2);
-                double s, c;
-                sincospi(2.0 * u2, &s, &c);
-                const double amp = unitary ? 1.0 : sqrt(-log(u1));
-                re = amp * c;
-                im = mirror ? -amp * s : amp * s;
+                ff t = wn_neg_log(v1);
+                if (self) t = ff_of(2.f * t.h, 2.f * t.l);
+                const ff amp = ff_sqrt(t);
+                re = ff_round_mul(amp, c);
+                im = ff_round_mul(amp, s);
             }
+            if (self) im = 0.f;
+            if (mirror) im = -im;
+            if (ij == 0 && l == 0) {
+                re = mean;
+                im = 0.f;
+            }
+            out[(long long)ij * zp + l] = make_float2(re, im);
         }
-        if (m == 0) {
-            re = mean;
-            im = 0.0;
-        }
-        out[ij * zp + l] = make_float2((float)re, (float)im);
     }
 }
 
@@ -1423,6 +1493,13 @@ void twiddle_table(std::vector<float2>& tw, int off, int n) {
     }
 }
 
+// sin(2 pi i / n), exact on the axes
+double table_sin(int i, int n) {
+    i %= n;
+    if ((4 * i) % n == 0) return (4 * i) / n == 1 ? 1.0 : (4 * i) / n == 3 ? -1.0 : 0.0;
+    return std::sin(2.0 * M_PI * (double)i / (double)n);
+}
+
 int device_init() {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return FPM_ERR_CUDA;
@@ -1446,6 +1523,21 @@ int device_init() {
     twiddle_table(tw, TwOff<1024>::v, 1024);
     twiddle_table(tw, TwOff<2048>::v, 2048);
     if (cudaMemcpyToSymbol(g_twiddle, tw.data(), sizeof(float2) * FPM_TW_TOTAL) != cudaSuccess)
+        return FPM_ERR_CUDA;
+    // the whitenoise tables
+    std::vector<float4> lg(128), tg(256);
+    for (int k = 0; k < 128; ++k) {
+        const float inv = k == 0 ? 1.f : k == 127 ? 0.5f : (float)(1.0 / (1.0 + (k + 0.5) / 128.0));
+        const int step = k >= 53 ? 1 : 0;   // f >= sqrt(2): u = 2^(e + 1) (f / 2)
+        const ff m = ff_split(-std::log((step ? 2.0 : 1.0) * (double)inv));
+        lg[k] = make_float4(inv, m.h, m.l, (float)step);
+    }
+    for (int k = 0; k < 256; ++k) {
+        const ff c = ff_split(table_sin(k + 64, 256)), sn = ff_split(table_sin(k, 256));
+        tg[k] = make_float4(c.h, c.l, sn.h, sn.l);
+    }
+    if (cudaMemcpyToSymbol(g_wn_log, lg.data(), 128 * sizeof(float4)) != cudaSuccess ||
+        cudaMemcpyToSymbol(g_wn_trig, tg.data(), 256 * sizeof(float4)) != cudaSuccess)
         return FPM_ERR_CUDA;
     g_init_done[dev] = true;
     return FPM_OK;
@@ -2473,14 +2565,11 @@ int fpm_whitenoise(void* cplx, int n, unsigned long long seed, int unitary, doub
     if (!fpm_fft_supported(n)) return FPM_ERR_SHAPE;
     int rc = device_init();
     if (rc) return rc;
-    const long long total = (long long)n * n * (n / 2 + 1);
-    const int threads = 256;
-    const long long blocks = (total + threads - 1) / threads;
+    const int blocks = (n * n + 7) / 8;   // a warp per row
     FPM_TRACE("whitenoise", (cudaStream_t)stream);
-    whitenoise_kernel<<<(unsigned)(blocks < 65535LL * 32 ? blocks : 65535LL * 32), threads, 0,
-                        (cudaStream_t)stream>>>((float2*)cplx, n, complex_row(n),
-                                                (uint32_t)(seed & 0xFFFFFFFFull),
-                                                (uint32_t)(seed >> 32), unitary, mean);
+    whitenoise_kernel<<<blocks < 152 * 64 ? blocks : 152 * 64, 256, 0, (cudaStream_t)stream>>>(
+        (float2*)cplx, n, complex_row(n), (uint32_t)(seed & 0xFFFFFFFFull), (uint32_t)(seed >> 32), unitary,
+        (float)mean);
     return fpm_launch_status();
 }
 
