@@ -1471,6 +1471,7 @@ __global__ void isotropic_kernel(float2* data, int n, int zp, const float* __res
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
+int fpm_internal_power_init();   // power.cu
 namespace {
 
 std::mutex g_init_mu;
@@ -1539,6 +1540,8 @@ int device_init() {
     if (cudaMemcpyToSymbol(g_wn_log, lg.data(), 128 * sizeof(float4)) != cudaSuccess ||
         cudaMemcpyToSymbol(g_wn_trig, tg.data(), 256 * sizeof(float4)) != cudaSuccess)
         return FPM_ERR_CUDA;
+    const int rc = fpm_internal_power_init();
+    if (rc) return rc;
     g_init_done[dev] = true;
     return FPM_OK;
 }

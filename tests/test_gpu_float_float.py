@@ -37,6 +37,37 @@ def _freq(n):
     return f.reshape(-1, 1, 1), f.reshape(1, -1, 1), numpy.arange(n // 2 + 1.0).reshape(1, 1, -1)
 
 
+# values in float32's middle, squares past float32's range on either side, and zeros
+@pytest.mark.parametrize('scale', [1.0, 1e-17, 1e-24, 1e15])
+@pytest.mark.parametrize('n', [16, 24, 96])
+def test_power_sums(G, n, scale):
+    pm, f1, v1 = _modes(G, n, n, scale)
+    _, f2, v2 = _modes(G, n, n + 1, scale)
+    f1.value[1, 2, 3] = 0
+    v1[1, 2, 3] = 0
+    fx, fy, fz = _freq(n)
+    q = fx ** 2 + fy ** 2 + fz ** 2
+    d = numpy.floor(numpy.sqrt(q)).astype(int)
+    w = numpy.where((fz == 0) | (fz == n // 2), 1.0, 2.0) * numpy.ones_like(q)
+    ok = d < n // 2
+    for other, vo in ((None, v1), (f2, v2)):
+        k, p, c = _sums(G, f1, other, n)
+        ref = [numpy.bincount(d[ok], weights=(x * w)[ok], minlength=n // 2)
+               for x in (numpy.sqrt(q) * (2 * numpy.pi / 50.0), abs(v1 * vo.conj()), numpy.ones_like(q))]
+        assert numpy.array_equal(c, ref[2])
+        # a float64 sum of m positive terms: m 2^-53 of it, m < 15000 here
+        numpy.testing.assert_allclose(k, ref[0], rtol=2e-12)
+        numpy.testing.assert_allclose(p, ref[1], rtol=2e-12)
+
+
+def test_power_not_finite(G):
+    n = 16
+    pm, f1, v1 = _modes(G, n, 3)
+    f1.value[2, 1, 0] = float('inf')   # shell 2
+    p = _sums(G, f1, None, n)[1]
+    assert not numpy.isfinite(p[2]) and numpy.isfinite(numpy.delete(p, 2)).all()
+
+
 @pytest.mark.parametrize('unitary', [False, True])
 @pytest.mark.parametrize('n', [16, 48])
 def test_whitenoise_rounds_as_float64(G, n, unitary):
