@@ -3,9 +3,14 @@
 // derivatives, and the k-space transfer transposes.  The chain rule they
 // implement is written out in fastpm-python_gb300/adjoint.py.
 #include "particles.cuh"
+#include "ff.cuh"
 #include "trace.h"
 
+#include <algorithm>
 #include <cmath>
+
+// fft.cu: the float64 sine table of mesh size n
+int fpm_internal_sin_table(int n, const double** table, int* stride);
 
 // ---------------------------------------------------------------------------
 // paint of per-particle values: mesh_m[cell] += scale * W * values_m[p * vstride_m]
@@ -120,6 +125,12 @@ __global__ void __launch_bounds__(256) readout_vjp_kernel(PartGeom g, VjpArgs a)
 // k-space combine on half meshes: out = scale * sum_m K_m(k) in_m(k) with
 //   K_m = (i a_x)^px (i a_y)^py (i a_z)^pz [/ k^2, 0 at k = 0, if lap_m]
 // a(k) = (8 sin kh - sin 2kh) / (6 h) (force/kernels.py:17-24).
+// The factors are float64 quantities applied to float32 modes.  In FP64 the six
+// sines and the divisions per mode bound the kernel (128^3, three inputs: 186
+// us); here a(k) comes from a float64 sine table, once per index and CTA, and
+// the factors, products and sums are float-float (ff.cuh, about 2^-44).
+// kspace_combine_f64_kernel keeps FP64 for scale factors outside float32's
+// comfortable range.
 // ---------------------------------------------------------------------------
 struct CombArgs {
     const float2* in[6];
@@ -129,14 +140,83 @@ struct CombArgs {
     float2* out;
     int n, zp;
     double inv6h, kf2, scale;
+    const double* sin_n;   // sin(2 pi i / n) = sin_n[i * sstride]
+    int sstride;
 };
 
-__device__ __forceinline__ double grad_a_exact(int i, int n, double inv6h) {
-    const double w = 2.0 * M_PI * (double)i / (double)n;
-    return (8.0 * sin(w) - sin(2.0 * w)) * inv6h;
+// (8 sin w - sin 2w) / (6 h) at w = 2 pi i / n, 0 <= i <= n/2
+__device__ __forceinline__ double grad_a_exact(const CombArgs& a, int i) {
+    return (8.0 * a.sin_n[i * a.sstride] - a.sin_n[(2 * i) % a.n * a.sstride]) * a.inv6h;
+}
+// multiply by i^ip
+__device__ __forceinline__ void comb_turn(int ip, float2& v) {
+    if (ip == 1) v = make_float2(-v.y, v.x);
+    else if (ip == 2) v = make_float2(-v.x, -v.y);
+    else if (ip == 3) v = make_float2(v.y, -v.x);
+}
+FPM_DEV ff ff_split_dev(double x) {
+    const float h = (float)x;
+    return ff{h, (float)(x - (double)h)};
 }
 
-__global__ void kspace_combine_kernel(CombArgs a) {
+// one mode in float64
+__device__ __noinline__ float2 comb_mode_f64(const CombArgs& a, int ni, int nj, int l, long long idx) {
+    const double ax = ni < 0 ? -grad_a_exact(a, -ni) : grad_a_exact(a, ni),
+                 ay = nj < 0 ? -grad_a_exact(a, -nj) : grad_a_exact(a, nj), az = grad_a_exact(a, l);
+    const long long q = (long long)ni * ni + (long long)nj * nj + (long long)l * l;
+    double re = 0.0, im = 0.0;
+    for (int s = 0; s < a.nin; ++s) {
+        double mag = 1.0;
+        for (int t = 0; t < a.pw[s][0]; ++t) mag *= ax;
+        for (int t = 0; t < a.pw[s][1]; ++t) mag *= ay;
+        for (int t = 0; t < a.pw[s][2]; ++t) mag *= az;
+        if (a.lap[s]) mag = q == 0 ? 0.0 : mag / (a.kf2 * (double)q);
+        float2 v = a.in[s][idx];
+        comb_turn((a.pw[s][0] + a.pw[s][1] + a.pw[s][2]) & 3, v);
+        re += v.x * mag;
+        im += v.y * mag;
+    }
+    return make_float2((float)(re * a.scale), (float)(im * a.scale));
+}
+
+// a warp per row (i, j), lanes along l
+__global__ void __launch_bounds__(256) kspace_combine_kernel(CombArgs a) {
+    __shared__ ff ga[513];   // a(k) of indices 0 .. n/2; a(-k) = -a(k)
+    const int n = a.n, nz = n / 2 + 1;
+    for (int i = threadIdx.x; i < nz; i += blockDim.x) ga[i] = ff_split_dev(grad_a_exact(a, i));
+    const ff kf2 = ff_split_dev(a.kf2), scale = ff_split_dev(a.scale);
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    for (int ij = blockIdx.x * 8 + (threadIdx.x >> 5); ij < n * n; ij += gridDim.x * 8) {
+        const int i = ij / n, j = ij - i * n;
+        const int ni = i < n / 2 ? i : i - n, nj = j < n / 2 ? j : j - n;
+        const ff ax = ni < 0 ? ff_neg(ga[-ni]) : ga[ni], ay = nj < 0 ? ff_neg(ga[-nj]) : ga[nj];
+        const int q2 = ni * ni + nj * nj;
+        for (int l = lane; l < nz; l += 32) {
+            const ff az = ga[l];
+            const int q = q2 + l * l;   // exact in float32 (at most 3 * 512^2)
+            const ff ilap = q == 0 ? ff_of(0.f) : ff_mul(scale, ff_recip(ff_mul_f(kf2, (float)q)));
+            const long long idx = (long long)ij * a.zp + l;
+            ff re = ff_of(0.f), im = ff_of(0.f);
+            for (int s = 0; s < a.nin; ++s) {
+                // (i ax)^px (i ay)^py (i az)^pz = i^(px+py+pz) ax^px ay^py az^pz
+                ff mag = a.lap[s] ? ilap : scale;
+                for (int t = 0; t < a.pw[s][0]; ++t) mag = ff_mul(mag, ax);
+                for (int t = 0; t < a.pw[s][1]; ++t) mag = ff_mul(mag, ay);
+                for (int t = 0; t < a.pw[s][2]; ++t) mag = ff_mul(mag, az);
+                float2 v = a.in[s][idx];
+                comb_turn((a.pw[s][0] + a.pw[s][1] + a.pw[s][2]) & 3, v);
+                re = ff_add(re, ff_mul_f(mag, v.x));
+                im = ff_add(im, ff_mul_f(mag, v.y));
+            }
+            // the error terms of an infinity are NaN: such a mode again in float64
+            a.out[idx] = isfinite(re.h) && isfinite(im.h) ? make_float2(re.h, im.h)
+                                                          : comb_mode_f64(a, ni, nj, l, idx);
+        }
+    }
+}
+
+__global__ void kspace_combine_f64_kernel(CombArgs a) {
     const int n = a.n, nz = n / 2 + 1;
     const long long total = (long long)n * n * nz;
     for (long long m = blockIdx.x * (long long)blockDim.x + threadIdx.x; m < total;
@@ -144,30 +224,8 @@ __global__ void kspace_combine_kernel(CombArgs a) {
         const int l = (int)(m % nz);
         const long long ij = m / nz;
         const int j = (int)(ij % n), i = (int)(ij / n);
-        const int ni = i < n / 2 ? i : i - n, nj = j < n / 2 ? j : j - n;
-        const double ax = grad_a_exact(ni, n, a.inv6h), ay = grad_a_exact(nj, n, a.inv6h),
-                     az = grad_a_exact(l, n, a.inv6h);
-        const long long q = (long long)ni * ni + (long long)nj * nj + (long long)l * l;
-        double re = 0.0, im = 0.0;
         const long long idx = ij * a.zp + l;
-        for (int s = 0; s < a.nin; ++s) {
-            // (i ax)^px (i ay)^py (i az)^pz = i^(px+py+pz) ax^px ay^py az^pz
-            double mag = 1.0;
-            for (int t = 0; t < a.pw[s][0]; ++t) mag *= ax;
-            for (int t = 0; t < a.pw[s][1]; ++t) mag *= ay;
-            for (int t = 0; t < a.pw[s][2]; ++t) mag *= az;
-            if (a.lap[s]) mag = q == 0 ? 0.0 : mag / (a.kf2 * (double)q);
-            const int ip = (a.pw[s][0] + a.pw[s][1] + a.pw[s][2]) & 3;
-            const float2 v = a.in[s][idx];
-            double vr = v.x * mag, vi = v.y * mag;
-            // multiply by i^ip
-            if (ip == 1) { const double t = vr; vr = -vi; vi = t; }
-            else if (ip == 2) { vr = -vr; vi = -vi; }
-            else if (ip == 3) { const double t = vr; vr = vi; vi = -t; }
-            re += vr;
-            im += vi;
-        }
-        a.out[idx] = make_float2((float)(re * a.scale), (float)(im * a.scale));
+        a.out[idx] = comb_mode_f64(a, i < n / 2 ? i : i - n, j < n / 2 ? j : j - n, l, idx);
     }
 }
 
@@ -297,10 +355,23 @@ int fpm_kspace_combine(const void* const* in, int nin, const int* powers, const 
     const double kf = 2.0 * M_PI / boxsize;
     a.kf2 = kf * kf;
     a.scale = scale;
+    int rc = fpm_internal_sin_table(n, &a.sin_n, &a.sstride);
+    if (rc) return rc;
     const long long total = (long long)n * n * (n / 2 + 1);
     cudaStream_t st = (cudaStream_t)stream;
     FPM_TRACE("kspace_combine", st);
-    kspace_combine_kernel<<<grid_for(total, 256), 256, 0, st>>>(a);
+    // the float-float form wants every factor, power and product of a normal
+    // size in float32: the widest range a mesh of 1024 cells and powers up to 2
+    // per axis spans is within 1e-12 .. 1e12 of these
+    auto tame = [](double x) { return x == 0.0 || (fabs(x) > 1e-6 && fabs(x) < 1e6); };
+    int deg = 0;
+    for (int s = 0; s < nin; ++s) deg = std::max(deg, a.pw[s][0] + a.pw[s][1] + a.pw[s][2]);
+    if (tame(a.inv6h) && tame(a.kf2) && tame(a.scale) && deg <= 2) {
+        const int blocks = (n * n + 7) / 8;
+        kspace_combine_kernel<<<blocks < 152 * 8 ? blocks : 152 * 8, 256, 0, st>>>(a);
+    } else {
+        kspace_combine_f64_kernel<<<grid_for(total, 256), 256, 0, st>>>(a);
+    }
     return fpm_launch_status();
 }
 

@@ -1468,6 +1468,10 @@ __global__ void isotropic_kernel(float2* data, int n, int zp, const float* __res
     }
 }
 
+// sin(2 pi i / 1024), then sin(2 pi i / 384), float64: every supported mesh size
+// divides one of the two
+static __device__ double g_sin64[1024 + 384];
+
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
@@ -1525,7 +1529,7 @@ int device_init() {
     twiddle_table(tw, TwOff<2048>::v, 2048);
     if (cudaMemcpyToSymbol(g_twiddle, tw.data(), sizeof(float2) * FPM_TW_TOTAL) != cudaSuccess)
         return FPM_ERR_CUDA;
-    // the whitenoise tables
+    // the whitenoise tables and the float64 sines of the k-space transfers
     std::vector<float4> lg(128), tg(256);
     for (int k = 0; k < 128; ++k) {
         const float inv = k == 0 ? 1.f : k == 127 ? 0.5f : (float)(1.0 / (1.0 + (k + 0.5) / 128.0));
@@ -1537,8 +1541,12 @@ int device_init() {
         const ff c = ff_split(table_sin(k + 64, 256)), sn = ff_split(table_sin(k, 256));
         tg[k] = make_float4(c.h, c.l, sn.h, sn.l);
     }
+    std::vector<double> sn(1024 + 384);
+    for (int i = 0; i < 1024; ++i) sn[i] = table_sin(i, 1024);
+    for (int i = 0; i < 384; ++i) sn[1024 + i] = table_sin(i, 384);
     if (cudaMemcpyToSymbol(g_wn_log, lg.data(), 128 * sizeof(float4)) != cudaSuccess ||
-        cudaMemcpyToSymbol(g_wn_trig, tg.data(), 256 * sizeof(float4)) != cudaSuccess)
+        cudaMemcpyToSymbol(g_wn_trig, tg.data(), 256 * sizeof(float4)) != cudaSuccess ||
+        cudaMemcpyToSymbol(g_sin64, sn.data(), sn.size() * sizeof(double)) != cudaSuccess)
         return FPM_ERR_CUDA;
     const int rc = fpm_internal_power_init();
     if (rc) return rc;
@@ -2238,6 +2246,19 @@ template <int N> struct Pipelines {
         case 1024: { constexpr int N = 1024; CALL; } \
         default: return FPM_ERR_SHAPE;   \
     }
+
+// the float64 sine table of mesh size n on this device: sin(2 pi i / n) is
+// (*table)[i * stride]
+int fpm_internal_sin_table(int n, const double** table, int* stride) {
+    int rc = device_init();
+    if (rc) return rc;
+    void* p = nullptr;
+    if (cudaGetSymbolAddress(&p, g_sin64) != cudaSuccess) return FPM_ERR_CUDA;
+    const bool two = 1024 % n == 0;
+    *table = (const double*)p + (two ? 0 : 1024);
+    *stride = (two ? 1024 : 384) / n;
+    return FPM_OK;
+}
 
 extern "C" {
 

@@ -76,3 +76,43 @@ def test_whitenoise_rounds_as_float64(G, n, unitary):
     for a, b in ((got.real, ref.real), (got.imag, ref.imag)):
         # half an ulp of the float32 result, and the 2^-36 of the float-float value (modulus up to about 6)
         assert (abs(a - b) <= 2.0 ** -24 * abs(b) * 1.01 + 6 * 2.0 ** -36).all()
+
+
+@pytest.mark.parametrize('scale', [-1.0, 1e-9])   # 1e-9: the FP64 form
+@pytest.mark.parametrize('n', [16, 24, 64, 96])
+def test_kspace_combine(G, n, scale):
+    from fastpm_gb300 import _lib
+    pw = [(1, 0, 0), (0, 1, 1), (0, 0, 2)]
+    lap = [1, 1, 0]
+    fields = [_modes(G, n, 7 + s) for s in range(3)]
+    pm = fields[0][0]
+    out = G.ComplexField(pm)
+    ptrs, keep = _lib.ptr_array([f[1].data for f in fields])
+    _lib.call('fpm_kspace_combine', ptrs, 3, (ctypes.c_int * 9)(*[x for p in pw for x in p]), (ctypes.c_int * 3)(*lap),
+              _lib.ptr(out.data), n, 50.0, scale, _lib.stream_ptr())
+    fx, fy, fz = _freq(n)
+    a = [(8 * numpy.sin(2 * numpy.pi * f / n) - numpy.sin(4 * numpy.pi * f / n)) * n / 300.0 for f in (fx, fy, fz)]
+    q = fx ** 2 + fy ** 2 + fz ** 2
+    k2 = numpy.where(q == 0, numpy.inf, q * (2 * numpy.pi / 50.0) ** 2)
+    ref, size = 0, 0
+    for (_, _, v), p, l in zip(fields, pw, lap):
+        t = scale * v * (1j * a[0]) ** p[0] * (1j * a[1]) ** p[1] * (1j * a[2]) ** p[2] / (k2 if l else 1.0)
+        ref, size = ref + t, size + abs(t)
+    # float32 rounding of the result; sin(pi) is 1e-16 in the reference, 0 in the table
+    err = abs(out.numpy() - ref)
+    assert (err <= 2.0 ** -23 * abs(ref) + 2.0 ** -40 * (size + abs(scale))).all()
+
+
+def test_kspace_combine_infinity(G):
+    from fastpm_gb300 import _lib
+    pm, f, v = _modes(G, 16, 1)
+    f.value[1, 1, 1] = complex(float('inf'), 1.0)
+    out = G.ComplexField(pm)
+    ptrs, keep = _lib.ptr_array([f.data])
+    _lib.call('fpm_kspace_combine', ptrs, 1, (ctypes.c_int * 3)(0, 0, 0), (ctypes.c_int * 1)(0), _lib.ptr(out.data), 16,
+              50.0, 2.0, _lib.stream_ptr())
+    got = out.numpy()
+    assert got[1, 1, 1] == complex(float('inf'), 2.0)
+    v[1, 1, 1] = 0
+    got[1, 1, 1] = 0
+    numpy.testing.assert_array_equal(got, (2 * v).astype('c8'))
