@@ -15,7 +15,13 @@
 
 #include "particles.cuh"
 
-template <int WINDOW>
+// Scatter paint: every window row (S consecutive z cells) goes out as vector
+// reductions of the one or two 16-byte quads it lies in, cells outside the
+// window adding 0.  The L2 takes one 16-byte reduction in the time of a 4-byte
+// one, so a TSC particle costs 9 to 18 of them instead of 27 (3 M clustered
+// particles on 256^3: 177 us; scalar 349 us).  Needs n a multiple of 4 and a
+// 16-byte aligned mesh (VEC); other meshes take scalar reductions.
+template <int WINDOW, bool VEC>
 __global__ void __launch_bounds__(256) paint_kernel(float* __restrict__ mesh_all, PartGeom g, float mass,
                                                     long long mesh_ss, long long disp_ss, const int* active) {
     if (active && !active[blockIdx.y]) return;
@@ -28,6 +34,7 @@ __global__ void __launch_bounds__(256) paint_kernel(float* __restrict__ mesh_all
         int cell[3][3];
         float w[3][3];
         particle_window<WINDOW>(g, p, cell, w);
+        const ZQuads<S> zq(cell[2][0], w[2], g.n);
 #pragma unroll
         for (int a = 0; a < S; ++a) {
             const float wa = w[0][a] * mass;
@@ -35,8 +42,12 @@ __global__ void __launch_bounds__(256) paint_kernel(float* __restrict__ mesh_all
             for (int b = 0; b < S; ++b) {
                 const float wab = wa * w[1][b];
                 float* row = mesh + ((long long)cell[0][a] * n + cell[1][b]) * n;
+                if (VEC) {
+                    zq.add(row, wab);
+                } else {
 #pragma unroll
-                for (int c = 0; c < S; ++c) atomicAdd(row + cell[2][c], wab * w[2][c]);
+                    for (int c = 0; c < S; ++c) atomicAdd(row + cell[2][c], wab * w[2][c]);
+                }
             }
         }
     }
@@ -58,12 +69,6 @@ struct TileGeom {
     int tz;       // tile edge in z, a multiple of 4
     int halo;     // cells of displacement spread tolerated around the mean
 };
-
-FPM_DEV void red_add_v4(float* addr, float a, float b, float c, float d) {
-    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b),
-                 "f"(c), "f"(d)
-                 : "memory");
-}
 
 template <int WINDOW>
 __global__ void __launch_bounds__(FPM_PAINT_THREADS)
@@ -959,7 +964,12 @@ struct ReadoutArgs {
     const int* active;
 };
 
-template <int WINDOW, int NM>
+// Readout of NM separate meshes in particle order.  VEC: a window row comes as
+// the one or two 16-byte quads it lies in instead of S scalar loads (a warp's
+// particles are spread over the mesh, so the loads' sectors are what counts: 3 M
+// particles on 256^3, TSC, one mesh: 132 us; scalar 160 us); needs n a multiple of
+// 4 and 16-byte aligned meshes.
+template <int WINDOW, int NM, bool VEC>
 __global__ void __launch_bounds__(256) readout_kernel(PartGeom g, ReadoutArgs r) {
     constexpr int S = Win<WINDOW>::S;
     const int slot = blockIdx.y;
@@ -979,18 +989,36 @@ __global__ void __launch_bounds__(256) readout_kernel(PartGeom g, ReadoutArgs r)
         float acc[NM];
 #pragma unroll
         for (int m = 0; m < NM; ++m) acc[m] = 0.f;
+        if (VEC) {
+            ZQuads<S> zq(cell[2][0], w[2], g.n);
 #pragma unroll
-        for (int a = 0; a < S; ++a) {
+            for (int a = 0; a < S; ++a) {
 #pragma unroll
-            for (int b = 0; b < S; ++b) {
-                const float wab = w[0][a] * w[1][b];
-                const long long rowoff = ((long long)cell[0][a] * n + cell[1][b]) * n;
+                for (int b = 0; b < S; ++b) {
+                    const float wab = w[0][a] * w[1][b];
+                    const long long row = ((long long)cell[0][a] * n + cell[1][b]) * n;
 #pragma unroll
-                for (int c = 0; c < S; ++c) {
-                    const float wt = wab * w[2][c];
-                    const long long idx = rowoff + cell[2][c];
+                    for (int m = 0; m < NM; ++m) {
+                        acc[m] += zq.template dot<0>(wab, __ldg(reinterpret_cast<const float4*>(r.mesh[m] + row + zq.q0)));
+                        if (zq.two)
+                            acc[m] += zq.template dot<4>(wab, __ldg(reinterpret_cast<const float4*>(r.mesh[m] + row + zq.q1)));
+                    }
+                }
+            }
+        } else {
 #pragma unroll
-                    for (int m = 0; m < NM; ++m) acc[m] += wt * __ldg(&r.mesh[m][idx]);
+            for (int a = 0; a < S; ++a) {
+#pragma unroll
+                for (int b = 0; b < S; ++b) {
+                    const float wab = w[0][a] * w[1][b];
+                    const long long rowoff = ((long long)cell[0][a] * n + cell[1][b]) * n;
+#pragma unroll
+                    for (int c = 0; c < S; ++c) {
+                        const float wt = wab * w[2][c];
+                        const long long idx = rowoff + cell[2][c];
+#pragma unroll
+                        for (int m = 0; m < NM; ++m) acc[m] += wt * __ldg(&r.mesh[m][idx]);
+                    }
                 }
             }
         }
@@ -1886,12 +1914,14 @@ int paint_impl(float* mesh, long long mesh_ss, int n, double boxsize, const floa
         return fpm_launch_status();
     }
     FPM_TRACE(window == FPM_WINDOW_CIC ? "paint_cic" : "paint_tsc", st);
-    if (window == FPM_WINDOW_CIC)
-        paint_kernel<FPM_WINDOW_CIC><<<dim3(grid_for(np, 256), nslot), 256, 0, st>>>(mesh, g, mass, mesh_ss,
-                                                                                   disp_ss, active);
-    else
-        paint_kernel<FPM_WINDOW_TSC><<<dim3(grid_for(np, 256), nslot), 256, 0, st>>>(mesh, g, mass, mesh_ss,
-                                                                                   disp_ss, active);
+    const bool vec = n % 4 == 0 && ((uintptr_t)mesh & 15) == 0 && mesh_ss % 4 == 0;
+#define FPM_SC(W, V) paint_kernel<W, V><<<dim3(grid_for(np, 256), nslot), 256, 0, st>>>(mesh, g, mass, mesh_ss, disp_ss, active)
+    if (window == FPM_WINDOW_CIC) {
+        if (vec) FPM_SC(FPM_WINDOW_CIC, true); else FPM_SC(FPM_WINDOW_CIC, false);
+    } else {
+        if (vec) FPM_SC(FPM_WINDOW_TSC, true); else FPM_SC(FPM_WINDOW_TSC, false);
+    }
+#undef FPM_SC
     return fpm_launch_status();
 }
 }  // namespace
@@ -2277,7 +2307,13 @@ int readout_impl(const float* const* meshes, long long mesh_ss, int nmesh, int n
     static const char* names[2][4] = {{"readout1_cic", "readout2_cic", "readout3_cic", "readout4_cic"},
                                       {"readout1_tsc", "readout2_tsc", "readout3_tsc", "readout4_tsc"}};
     FPM_TRACE(names[window == FPM_WINDOW_TSC][nmesh - 1], st);
-#define FPM_RO(W, NM) readout_kernel<W, NM><<<dim3(grid, nslot), 256, 0, st>>>(g, r)
+    bool vec = n % 4 == 0 && mesh_ss % 4 == 0;
+    for (int m = 0; m < nmesh; ++m) vec = vec && ((uintptr_t)meshes[m] & 15) == 0;
+#define FPM_RO(W, NM)                                                              \
+    do {                                                                           \
+        if (vec) readout_kernel<W, NM, true><<<dim3(grid, nslot), 256, 0, st>>>(g, r); \
+        else readout_kernel<W, NM, false><<<dim3(grid, nslot), 256, 0, st>>>(g, r);    \
+    } while (0)
     if (window == FPM_WINDOW_CIC) {
         switch (nmesh) {
             case 1: FPM_RO(FPM_WINDOW_CIC, 1); break;

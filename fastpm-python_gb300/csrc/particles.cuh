@@ -140,6 +140,50 @@ FPM_DEV void particle_window(const PartGeom& g, long long p, int (*cell)[3], flo
     }
 }
 
+FPM_DEV void red_add_v4(float* addr, float a, float b, float c, float d) {
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b),
+                 "f"(c), "f"(d)
+                 : "memory");
+}
+
+// The S z cells from z0 of a window row as aligned quads of four cells (n a
+// multiple of 4): they lie in the quad at q0 and, when two, the next one at q1
+// (wrapped).  w[j] is the weight of cell q0 + j, in(j) whether it is in the
+// window: what lies outside it must not count, be it infinite.
+template <int S> struct ZQuads {
+    int q0, q1, k;
+    bool two;
+    float w[7];
+    FPM_DEV ZQuads(int z0, const float* wz, int n) {
+        k = z0 & 3;
+        q0 = z0 - k;
+        q1 = q0 + 4 == n ? 0 : q0 + 4;
+        two = k + S > 4;
+#pragma unroll
+        for (int j = 0; j < 7; ++j) {
+            float v = 0.f;
+#pragma unroll
+            for (int s = 0; s < S; ++s)
+                if (j >= s && j - s < 4) v = k == j - s ? wz[s] : v;
+            w[j] = v;
+        }
+    }
+    FPM_DEV bool in(int j) const { return (unsigned)(j - k) < (unsigned)S; }
+    // sum of wab w[j] v[j] over the window's cells of the quad J = 0 or 4
+    template <int J> FPM_DEV float dot(float wab, float4 v) const {
+        const float* c = reinterpret_cast<const float*>(&v);
+        float s = 0.f;
+#pragma unroll
+        for (int j = 0; j < (J ? 3 : 4); ++j) s += in(J + j) ? (wab * w[J + j]) * c[j] : 0.f;
+        return s;
+    }
+    FPM_DEV float at(float wab, int j) const { return in(j) ? wab * w[j] : 0.f; }
+    // row[cell] += wab w[cell] over the window: one or two vector reductions
+    FPM_DEV void add(float* row, float wab) const {
+        red_add_v4(row + q0, at(wab, 0), at(wab, 1), at(wab, 2), at(wab, 3));
+        if (two) red_add_v4(row + q1, at(wab, 4), at(wab, 5), at(wab, 6), 0.f);
+    }
+};
 
 // window derivative along one axis (per cell unit)
 template <int WINDOW> struct WinGrad;
