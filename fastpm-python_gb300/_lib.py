@@ -60,6 +60,9 @@ SIGNATURES = {
     'fpm_force_mesh_static': (_i, [_vp, _i, _d, _d, _d, _vp, _vp, _vp, _vp, _vp]),
     'fpm_whitenoise': (_i, [_vp, _i, _u64, _i, _d, _vp]),
     'fpm_apply_isotropic': (_i, [_vp, _i, _vp, _ll, _vp]),
+    'fpm_apply_isotropic_to': (_i, [_vp, _vp, _i, _vp, _ll, _vp]),
+    'fpm_lpt_readout': (_i, [_pp, _i, _d, _vp, _ll, _i, _d, _vp, _vp, _vp, _vp, _vp,
+                             _c.POINTER(_d), _c.POINTER(_d), _vp]),
     'fpm_kick': (_i, [_vp, _vp, _vp, _ll, _d, _vp]),
     'fpm_drift': (_i, [_vp, _vp, _vp, _ll, _d, _vp]),
     'fpm_kick_drift': (_i, [_vp, _vp, _vp, _vp, _vp, _ll, _d, _d, _i, _d, _vp]),

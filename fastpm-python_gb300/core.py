@@ -30,7 +30,8 @@ def _is_cosmology(c):
 class StateVector(object):
     """fastpm/core.py:7-89."""
 
-    def __init__(self, solver, Q):
+    def __init__(self, solver, Q, _unset=False):
+        # _unset: S, P and F are left unset for a caller that writes all of them
         self.solver = solver
         self.pm = solver.pm
         device = solver.pm.device
@@ -51,9 +52,10 @@ class StateVector(object):
         self.q32 = None if lat is not None else Q.to(device=device, dtype=torch.float32).contiguous()
         np_ = len(Q)
         z = lambda *s: torch.zeros(*s, dtype=torch.float32, device=device)
-        self.S = z(np_, 3)
-        self.P = z(np_, 3)
-        self.F = z(np_, 3)
+        zs = (lambda *s: torch.empty(*s, dtype=torch.float32, device=device)) if _unset else z
+        self.S = zs(np_, 3)
+        self.P = zs(np_, 3)
+        self.F = zs(np_, 3)
         self.RHO = z(np_)
         # Kahan compensation of S and P, bfloat16 (the kernels' storage format)
         self.S_c = torch.zeros(np_, 3, dtype=torch.bfloat16, device=device)
@@ -137,9 +139,9 @@ class Solver(object):
         # pinned and asynchronous: a pageable copy would make the host wait for
         # everything queued on the stream before it
         t = torch.from_numpy(table.astype('f4')).pin_memory().to(pm.device, non_blocking=True)
-        out = whitenoise.copy()
-        _lib.call('fpm_apply_isotropic', _lib.ptr(out.data), n, _lib.ptr(t), len(table),
-                  _lib.stream_ptr())
+        out = ComplexField(pm, empty=True)
+        _lib.call('fpm_apply_isotropic_to', _lib.ptr(whitenoise.data), _lib.ptr(out.data), n, _lib.ptr(t),
+                  len(table), _lib.stream_ptr())
         return out
 
     def lpt(self, linear, Q, a, order=2):
@@ -152,23 +154,15 @@ class Solver(object):
         waiting for the stream here; growth: a MatterDominated of this
         cosmology (normalised at a_linear) already solved on a grid holding a."""
         assert order in (1, 2)
-        from .force import lpt1, lpt2source
-        state = StateVector(self, Q)
+        from .force import lpt_state
+        state = StateVector(self, Q, _unset=True)
         pt = growth if growth is not None else MatterDominated(self.cosmology.Om0, a=[a],
                                                                a_normalize=self.a_linear)
         D1, D2 = float(pt.D1(a)), float(pt.D2(a))
         f1, f2, E = float(pt.f1(a)), float(pt.f2(a)), float(pt.E(a))
         gf, gf2 = float(pt.gf(a)), float(pt.gf2(a))
-        dx1 = lpt1(linear, state)
-        if order == 2:
-            dx2 = lpt1(lpt2source(linear), state)
-            state.S[...] = D1 * dx1 + D2 * dx2
-            state.P[...] = (a ** 2 * f1 * E * D1) * dx1 + (a ** 2 * f2 * E * D2) * dx2
-            state.F[...] = (a ** 2 * E * gf) * dx1 + (a ** 2 * E * gf2) * dx2
-        else:
-            state.S[...] = D1 * dx1
-            state.P[...] = (a ** 2 * f1 * E * D1) * dx1
-            state.F[...] = (a ** 2 * E * gf) * dx1
+        lpt_state(linear, state, order, (D1, a ** 2 * f1 * E * D1, a ** 2 * E * gf),
+                  (D2, a ** 2 * f2 * E * D2, a ** 2 * E * gf2))
         state.a['S'] = a
         state.a['P'] = a
         work = self.pm._bufs.get('lpt_ws')

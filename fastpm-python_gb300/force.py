@@ -1,5 +1,7 @@
 """fastpm.force on the device: lpt1 / lpt2source (force/lpt.py) and the
 long-range PM force (force/gravity.py:5-29) as fused mesh pipelines."""
+import ctypes
+
 import torch
 
 from . import _lib
@@ -11,6 +13,25 @@ def _lpt_work(pm):
     return pm._scratch('lpt_ws', nbytes), nbytes
 
 
+def _lpt1_meshes(dlin_k):
+    """The three displacement meshes c2r(i a_d lap dlin_k) in pm's scratch."""
+    pm = dlin_k.pm
+    n = pm.n
+    work, nbytes = _lpt_work(pm)
+    meshes = pm._scratch('lpt_mesh', 3 * n ** 3 * 4).view(torch.float32).view(3, n, n, n)
+    _lib.call('fpm_lpt1_mesh', _lib.ptr(dlin_k.data), n, pm.L, _lib.ptr(meshes[0]),
+              _lib.ptr(meshes[1]), _lib.ptr(meshes[2]), _lib.ptr(work), nbytes, _lib.stream_ptr())
+    return meshes
+
+
+def _lpt_readout(pm, meshes, state, psi1=None, psi_out=None, out=(None, None, None), c1=None, c2=None):
+    qp, np_, nc, shift = pm._geom(state.q32, None, state.lattice)
+    m_arr, _keep = _lib.ptr_array([meshes[0], meshes[1], meshes[2]])
+    three = lambda c: (ctypes.c_double * 3)(*c) if c is not None else None
+    _lib.call('fpm_lpt_readout', m_arr, pm.n, pm.L, qp, np_, nc, shift, _lib.ptr(psi1), _lib.ptr(psi_out),
+              _lib.ptr(out[0]), _lib.ptr(out[1]), _lib.ptr(out[2]), three(c1), three(c2), _lib.stream_ptr())
+
+
 def lpt1(dlin_k, state, resampler='cic'):
     """force/lpt.py:4-23: psi_d = readout_CIC(c2r(i a_d lap dlin_k)) at the state's Q.
 
@@ -18,15 +39,27 @@ def lpt1(dlin_k, state, resampler='cic'):
     Returns float32 [Np, 3] on the device.
     """
     pm = dlin_k.pm
-    n = pm.n
-    work, nbytes = _lpt_work(pm)
-    meshes = pm._scratch('lpt_mesh', 3 * n ** 3 * 4).view(torch.float32).view(3, n, n, n)
-    _lib.call('fpm_lpt1_mesh', _lib.ptr(dlin_k.data), n, pm.L, _lib.ptr(meshes[0]),
-              _lib.ptr(meshes[1]), _lib.ptr(meshes[2]), _lib.ptr(work), nbytes, _lib.stream_ptr())
+    meshes = _lpt1_meshes(dlin_k)
     out = torch.empty((state.csize, 3), dtype=torch.float32, device=pm.device)
-    pm._readout([meshes[0], meshes[1], meshes[2]], [out[:, 0], out[:, 1], out[:, 2]], [3, 3, 3],
-                [1.0, 1.0, 1.0], q=state.q32, disp=None, lattice=state.lattice, resampler=resampler)
+    if resampler == 'cic':
+        _lpt_readout(pm, meshes, state, psi_out=out)
+    else:
+        pm._readout([meshes[0], meshes[1], meshes[2]], [out[:, 0], out[:, 1], out[:, 2]], [3, 3, 3],
+                    [1.0, 1.0, 1.0], q=state.q32, disp=None, lattice=state.lattice, resampler=resampler)
     return out
+
+
+def lpt_state(dlin_k, state, order, c1, c2):
+    """S, P and F of `state` from the displacements of the linear field:
+    c1[k] psi1, or with order 2 c1[k] psi1 + c2[k] psi2 (core.py:128-145), the
+    second readout writing the state directly."""
+    pm = dlin_k.pm
+    out = (state.S, state.P, state.F)
+    if order == 1:
+        _lpt_readout(pm, _lpt1_meshes(dlin_k), state, out=out, c1=c1)
+        return
+    psi1 = lpt1(dlin_k, state)
+    _lpt_readout(pm, _lpt1_meshes(lpt2source(dlin_k)), state, psi1=psi1, out=out, c1=c1, c2=c2)
 
 
 def lpt2source(dlin_k):

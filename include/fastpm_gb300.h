@@ -313,6 +313,14 @@ long long fpm_lpt_workspace(int n);
 int fpm_lpt1_mesh(const void* dlin_k, int n, double boxsize,
                   float* disp_x, float* disp_y, float* disp_z,
                   void* work, long long work_bytes, void* stream);
+/* The particle part of force/lpt.py:4-23 and of the 2LPT state
+ * (core.py:128-145): x = CIC readout of meshes[0..2] (host array) at the
+ * lattice points (q == NULL) or at q.  psi_out: x itself, [np][3].  Else the
+ * state, k = 0, 1, 2 for s, p, f: c1[k] psi1 + c2[k] x with psi1 an earlier
+ * readout [np][3], or c1[k] x when psi1 is NULL (c1, c2: host arrays of 3).   */
+int fpm_lpt_readout(const float* const* meshes, int n, double boxsize, const float* q, long long np,
+                    int nc, double shift, const float* psi1, float* psi_out, float* s, float* p,
+                    float* f, const double* c1, const double* c2, void* stream);
 /* Allocation-free fpm_force_mesh (no counterpart in the reference): for
  * callers that cannot allocate device memory where they need a force, e.g. a
  * host with a fixed device-memory budget, or one that must not let
@@ -355,6 +363,9 @@ int fpm_whitenoise(void* cplx, int n, unsigned long long seed, int unitary, doub
  * q = 0 .. 3 (n/2)^2 (table_len entries, float32, device memory).           */
 int fpm_apply_isotropic(void* cplx, int n, const float* table, long long table_len,
                         void* stream);
+/* The same out of place, out = in * table (one pass; out may be in).        */
+int fpm_apply_isotropic_to(const void* in, void* out, int n, const float* table,
+                           long long table_len, void* stream);
 
 /* ---- time stepping --------------------------------------------------------
  * replaces fastpm/core.py:168-173 (Kick: P += fac F) and 175-180 (Drift:
