@@ -1114,6 +1114,86 @@ grad_stencil(const float* __restrict__ phi, float* __restrict__ fx, float* __res
     }
 }
 
+// The same without shared memory or barriers: a thread forms four z cells (one
+// 16-byte load per neighbour quad) of XR consecutive planes, keeping its x
+// neighbours in registers; y and z neighbours and the halos come through L1 and
+// L2, every load of a plane independent of the others.  The ring kernel above
+// waits at two barriers per plane with two planes in flight: 4897 us at n = 1024
+// (packed) against 3848 here, 0.99 of the measured HBM copy rate for its 24 B per
+// cell; n = 512 635 -> 490, 256 90.6 -> 67.7, 128 25.8 -> 14.2, 64 20.4 -> 7.9.
+// XR planes per thread: 1 fills the chip best below n = 512 (n = 384: 211 us with
+// 1, 213 with 2, 231 with 4), 2 above (n = 1024: 3875 / 3848 / 4257).
+// Needs 16-byte aligned phi, rho and outputs (the packed mesh 32-byte, for 256-bit
+// stores); other arrays take the ring kernel.
+FPM_DEV void st_pair(float4* p, float4 a, float4 b) {   // two cells with one 256-bit store
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z),
+                 "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+                 : "memory");
+}
+template <int N> struct StenD {
+    static constexpr int XR = N < 512 ? 1 : 2;
+    static constexpr int ZQ = N / 4 < 32 ? N / 4 : 32;   // z quads per CTA row
+    static constexpr int YR = 256 / ZQ < N ? 256 / ZQ : N;
+    static constexpr int THREADS = ZQ * YR;
+    static constexpr int NZB = (N / 4 + ZQ - 1) / ZQ, NYB = (N + YR - 1) / YR;
+};
+template <int N, int PACK, int XR>
+__global__ void __launch_bounds__(StenD<N>::THREADS)
+grad_direct(const float* __restrict__ phi, float* __restrict__ fx, float* __restrict__ fy, float* __restrict__ fz,
+            float c, const float* __restrict__ rho, float4* __restrict__ packed, float rs, long long phi_ss,
+            long long rho_ss, long long packed_ss, const int* __restrict__ active,
+            const float* __restrict__ slot_coef) {
+    using S = StenD<N>;
+    if (active && !active[blockIdx.y]) return;
+    if (PACK) {
+        phi += blockIdx.y * phi_ss;
+        rho += blockIdx.y * rho_ss;
+        packed += blockIdx.y * packed_ss;
+        if (slot_coef) c *= slot_coef[blockIdx.y];
+    }
+    const int zq = (blockIdx.x % S::NZB) * S::ZQ + threadIdx.x % S::ZQ;
+    const int y = (blockIdx.x / S::NZB) * S::YR + threadIdx.x / S::ZQ;
+    if (zq >= N / 4 || y >= N) return;
+    const int z = 4 * zq, zl = (z + N - 4) % N, zr = (z + 4) % N;
+    auto row = [&](int yy) { return ((yy + N) % N) * N; };
+    const int rm2 = row(y - 2) + z, rm1 = row(y - 1) + z, rp1 = row(y + 1) + z, rp2 = row(y + 2) + z, r0 = y * N;
+    auto plane = [&](int x) { return phi + (long long)((x + N) % N) * N * N; };
+    auto q4 = [](const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); };
+    const int x0 = blockIdx.z * XR;
+    float4 v[XR + 4];
+#pragma unroll
+    for (int i = 0; i < XR + 4; ++i) v[i] = q4(plane(x0 - 2 + i) + r0 + z);
+#pragma unroll
+    for (int i = 0; i < XR; ++i) {
+        const float* p = plane(x0 + i);
+        const float4 ym2 = q4(p + rm2), ym1 = q4(p + rm1), yp1 = q4(p + rp1), yp2 = q4(p + rp2);
+        const float4 l = q4(p + r0 + zl), r = q4(p + r0 + zr);
+        const long long o = ((long long)(x0 + i) * N + y) * N + z;
+        const float4 rh = PACK ? __ldcs(reinterpret_cast<const float4*>(rho + o)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 c0 = v[i + 2];
+        const float w[8] = {l.z, l.w, c0.x, c0.y, c0.z, c0.w, r.x, r.y};   // z - 2 .. z + 5
+        auto at = [](const float4& f, int k) { return k == 0 ? f.x : k == 1 ? f.y : k == 2 ? f.z : f.w; };
+        float dx[4], dy[4], dz[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            dx[k] = (8.f * (at(v[i + 3], k) - at(v[i + 1], k)) - (at(v[i + 4], k) - at(v[i], k))) * c;
+            dy[k] = (8.f * (at(yp1, k) - at(ym1, k)) - (at(yp2, k) - at(ym2, k))) * c;
+            dz[k] = (8.f * (w[k + 3] - w[k + 1]) - (w[k + 4] - w[k])) * c;
+        }
+        if (PACK) {
+#pragma unroll
+            for (int k = 0; k < 4; k += 2)
+                st_pair(packed + (PACK == 2 ? blocked_cell(N, x0 + i, y, z + k) : o + k),
+                        make_float4(dx[k], dy[k], dz[k], at(rh, k) * rs),
+                        make_float4(dx[k + 1], dy[k + 1], dz[k + 1], at(rh, k + 1) * rs));
+        } else {
+            __stcs(reinterpret_cast<float4*>(fx + o), make_float4(dx[0], dx[1], dx[2], dx[3]));
+            __stcs(reinterpret_cast<float4*>(fy + o), make_float4(dy[0], dy[1], dy[2], dy[3]));
+            __stcs(reinterpret_cast<float4*>(fz + o), make_float4(dz[0], dz[1], dz[2], dz[3]));
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Plane-batched persistent kernels (n >= 512).  Work items are handed out in
 // order from a global counter: for x-plane batch b, first the phase-1 items
@@ -1806,6 +1886,18 @@ template <int N> int launch_stencil(const float* phi, float* fx, float* fy, floa
                                     const float* slot_coef = nullptr, bool blocked = false) {
     using S = Sten<N>;
     const float c = (float)((double)N / (12.0 * boxsize));   // 1 / (12 h)
+    const uintptr_t low = packed ? (((uintptr_t)phi | (uintptr_t)rho) & 15) | ((uintptr_t)packed & 31) |
+                                       (uintptr_t)((phi_ss | rho_ss) & 3) | (uintptr_t)(packed_ss & 1)
+                                 : ((uintptr_t)phi | (uintptr_t)fx | (uintptr_t)fy | (uintptr_t)fz) & 15;
+    if (low == 0) {
+        using D = StenD<N>;
+        constexpr int XR = D::XR;
+        auto kern = packed ? (blocked ? grad_direct<N, 2, XR> : grad_direct<N, 1, XR>) : grad_direct<N, 0, XR>;
+        FPM_TRACE("grad_stencil", st);
+        kern<<<dim3(D::NZB * D::NYB, nslot, N / XR), D::THREADS, 0, st>>>(phi, fx, fy, fz, c, rho, packed, rs, phi_ss,
+                                                                        rho_ss, packed_ss, active, slot_coef);
+        return fpm_launch_status();
+    }
     // split the x sweep into segments so the launch is at least ~8 waves of
     // resident CTAs (each segment reloads its 4 halo planes)
     const long long cols = (long long)(N / S::BY) * (N / S::BZ) * nslot;
