@@ -277,14 +277,15 @@ FPM_DEV void decode_bkey(unsigned key, int nb, int (*bk)[2], bool* two) {
 // counting pass stores the particle id straight into its home brick's bucket
 // (capacity ch) and each window tail into the tail brick's bucket (capacity
 // ct).  An id past a full bucket goes to the spill list; if that overflows
-// too, the mode word becomes 2 and the paint rebuilds the lists the classic
-// way (recount and fill).
+// too, the mode word becomes 2 and the paint places the ids itself
+// (bin_place_kernel).
 struct Buckets {
     int* home;   // [brick][ch]
     int* tail;   // [brick][ct]
     int ch, ct;  // bucket strides
     int lh, lt;  // entries a bucket may hold (<= ch, ct)
     int* mode;   // 0: buckets valid, 2: the spill list overflowed
+    int* limits; // lh, lt for the paint that reads the buckets
     int2* spill; // entries past a full bucket: (brick | 2^30 for a tail, id)
     int* nspill;
     int spill_cap;
@@ -405,24 +406,12 @@ FPM_DEV void bin_warp_count(bool live, long long p, const int (*bk)[2], const bo
 // particle's brick key and home rank kept for the fill (grid y = slot;
 // per-slot arrays sit bg.stride ints (counters) and np ints (keys, ranks)
 // apart, displacements disp_ss floats apart)
-// After an overflowed bucket (mode word 2): zero the brick counts, which the
-// fused kick-drift left holding its totals, before the paint recounts.
-__global__ void __launch_bounds__(256) bucket_overflow_reset_kernel(const int* __restrict__ mode,
-                                                                    int* __restrict__ counts, long long len) {
-    if (*mode != 2) return;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += (long long)gridDim.x * blockDim.x)
-        counts[i] = 0;
-}
-
 template <int WINDOW, int LOGBS>
 __global__ void __launch_bounds__(256) bin_count_kernel(PartGeom g, BrickGeom bg, int* __restrict__ count,
                                                         int* __restrict__ hcount, int* __restrict__ hrank,
                                                         unsigned* __restrict__ keys, long long disp_ss,
-                                                        const int* __restrict__ active,
-                                                        const int* __restrict__ run_if = nullptr) {
+                                                        const int* __restrict__ active) {
     if (active && !active[blockIdx.y]) return;
-    // run_if: the mode word of bucketed lists; recount only after an overflow
-    if (run_if && *run_if != 2) return;
     count += blockIdx.y * (long long)bg.stride;
     hcount += blockIdx.y * (long long)bg.stride;
     hrank += blockIdx.y * g.np;
@@ -463,11 +452,8 @@ __global__ void __launch_bounds__(256) bin_fill_kernel(const unsigned* __restric
                                                        const int* __restrict__ hrank, long long np,
                                                        BrickGeom bg, const int* __restrict__ off,
                                                        int* __restrict__ back, int* __restrict__ entries,
-                                                       const int* __restrict__ active,
-                                                       const int* __restrict__ mode = nullptr) {
+                                                       const int* __restrict__ active) {
     if (active && !active[blockIdx.y]) return;
-    // mode: the mode word of bucketed lists; valid buckets: the deposit copies them
-    if (mode && *mode == 0) return;
     off += blockIdx.y * (long long)bg.stride;
     back += blockIdx.y * (long long)bg.stride;
     entries += blockIdx.y * 8 * np;
@@ -488,6 +474,61 @@ __global__ void __launch_bounds__(256) bin_fill_kernel(const unsigned* __restric
             entries[__ldg(off + home) + __ldg(hrank + p)] = (int)p;
         }
         bin_warp_tails<1>(live, p, bk, two, lane, nb, nullptr, back, entries, items[threadIdx.x >> 5]);
+    }
+}
+
+// The lists of a paint whose counts came from the fused kick-drift but whose
+// buckets do not hold them (mode word not 0: option 26 off, or the spill list
+// overflowed): the positions' bricks again, each run of homes taking its ranks from
+// hcount downwards (the deposit puts the totals back), the tails from the back
+// cursors.  With valid buckets it returns at once, so its grid is small: it and the
+// scan are all that runs between kick-drift and deposit (a reset, a recount and a
+// fill launched over the particles before: 11 to 25 us per step).
+template <int WINDOW, int LOGBS>
+__global__ void __launch_bounds__(256) bin_place_kernel(PartGeom g, BrickGeom bg, const int* __restrict__ mode,
+                                                        const int* __restrict__ off, int* __restrict__ hcount,
+                                                        int* __restrict__ back, int* __restrict__ entries) {
+    if (*mode == 0) return;
+    constexpr int S = Win<WINDOW>::S;
+    const unsigned full = 0xffffffffu;
+    __shared__ int2 items[8][256];
+    const int lane = threadIdx.x & 31;
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long base = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < g.np; base += stride) {
+        const long long p = base + lane;
+        const bool live = p < g.np;
+        int bk[3][2] = {{0, 0}, {0, 0}, {0, 0}};
+        bool two[3] = {false, false, false};
+        int key = -1;
+        if (live) {
+            int c0[3];
+            window_first_cells<WINDOW>(g, p, c0);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                int last = c0[d] + S - 1;
+                if (last >= g.n) last -= g.n;
+                bk[d][0] = c0[d] >> LOGBS;
+                bk[d][1] = last >> LOGBS;
+                two[d] = bk[d][1] != bk[d][0];
+            }
+            key = (bk[0][0] * bg.nb + bk[1][0]) * bg.nb + bk[2][0];
+        }
+        // the run's ranks with one atomic, as in bin_warp_home_ranks
+        const unsigned livem = __ballot_sync(full, live);
+        const int prev = __shfl_up_sync(full, key, 1);
+        const bool head = live && (lane == 0 || prev != key);
+        const unsigned heads = __ballot_sync(full, head), upto = (2u << lane) - 1u;
+        int pos = 0;
+        if (head) {
+            const unsigned after = (heads | ~livem) & ~upto;
+            const int len = (after ? __ffs(after) - 1 : 32) - lane;
+            pos = off[key] + atomicSub(hcount + key, len) - len;
+        }
+        const unsigned mine = heads & upto;
+        const int h = mine ? 31 - __clz(mine) : 0;
+        pos = __shfl_sync(full, pos, h);
+        if (live) entries[pos + lane - h] = (int)p;
+        bin_warp_tails<1>(live, p, bk, two, lane, bg.nb, nullptr, back, entries, items[threadIdx.x >> 5]);
     }
 }
 
@@ -802,6 +843,8 @@ FPM_DEV void brick_deposit(void* tile, const PartGeom& g, const int* __restrict_
 // (homes at off[b], tails after them) for the readouts that follow.
 struct BucketLists {
     const int* mode;
+    const int* limits;
+    int* hcount;
     const int* home;
     const int* tail;
     const int* cursor;
@@ -846,9 +889,11 @@ __global__ void __launch_bounds__(256, FPM_PAINT_MINB) paint_brick_kernel(float*
     const bool bucketed = bl.mode != nullptr && *bl.mode == 0;
     const int nhome = bucketed ? bl.cursor[b] - e0 : e1 - e0;   // homes in all
     const int ntail = e1 - e0 - nhome;
-    // the limits the kick-drift filled the buckets to (mode word block)
-    const int nh = bucketed ? min(nhome, bl.mode[1]) : nhome;   // from r0
-    const int nt = bucketed ? min(ntail, bl.mode[2]) : ntail;   // from r1
+    // the limits the kick-drift filled the buckets to
+    const int nh = bucketed ? min(nhome, bl.limits[0]) : nhome;   // from r0
+    const int nt = bucketed ? min(ntail, bl.limits[1]) : ntail;   // from r1
+    // bin_place_kernel took the home ranks from hcount: its total again
+    if (bl.mode != nullptr && !bucketed && threadIdx.x == 0) bl.hcount[b] = bl.cursor[b] - e0;
     const int* r0 = bucketed ? bl.home + (long long)b * bl.ch : entries + e0;
     const int* r1 = bucketed ? bl.tail + (long long)b * bl.ct : entries + e0 + nhome;
     // spilled entries of this brick, in the list: homes at [e0 + nh, e0 + nhome),
@@ -1864,8 +1909,8 @@ __global__ void __launch_bounds__(256) kick_drift_bin_kernel(float* __restrict__
     constexpr int S = Win<WINDOW>::S;
     // the bucket limits, for the paint that reads the buckets
     if (BUCKET && blockIdx.x == 0 && threadIdx.x == 0) {
-        bkt.mode[1] = bkt.lh;
-        bkt.mode[2] = bkt.lt;
+        bkt.limits[0] = bkt.lh;
+        bkt.limits[1] = bkt.lt;
     }
     __shared__ __align__(16) float vsh[VEC ? 8 : 1][VEC ? 96 : 4];   // per warp: 32 new positions
     __shared__ int2 items[8][256];
@@ -2047,7 +2092,8 @@ struct SortedWork {
     int pstride;      // ints per slot in part
     // single-slot workspaces only (NULL / 0 otherwise): the mode word and the
     // bucketed lists of the fused kick-drift (Buckets)
-    int* mode;
+    int* mode;        // in the spare entry past count's last brick (nspill past hcount's): one
+    int* limits;      // memset zeroes the counts and both words
     int* bucket_h;
     int* bucket_t;
     int ch, ct;
@@ -2105,13 +2151,14 @@ SortedWork sorted_layout(char* base, int n, long long np, int nslot, int bs, boo
     o += up((long long)nslot * np * 4);
     w.entries = (int*)(base + o);
     o += up((long long)nslot * 8 * np * 4);
-    w.mode = w.bucket_h = w.bucket_t = w.nspill = nullptr;
+    w.mode = w.limits = w.bucket_h = w.bucket_t = w.nspill = nullptr;
     w.spill = nullptr;
     w.ch = w.ct = w.spill_cap = 0;
     if (buckets && nslot == 1 && nbrick > 0) {
         bucket_caps(np, nbrick, w.ch, w.ct);
-        w.mode = (int*)(base + o);
-        w.nspill = w.mode + 32;
+        w.mode = w.count + nbrick;     // stride > nbrick
+        w.nspill = w.hcount + nbrick;
+        w.limits = (int*)(base + o);
         o += 256;
         w.bucket_h = (int*)(base + o);
         o += up(nbrick * w.ch * 4LL);
@@ -2164,35 +2211,34 @@ int paint_sorted_impl(float* mesh, long long mesh_ss, int n, double boxsize, con
         return FPM_ERR_CUDA;
     // the mode word of a single-slot workspace: a paint that counts for
     // itself builds the classic lists; after the fused kick-drift the word
-    // says whether its buckets hold the lists (0), overflowed (2: recount
-    // here) or were not used (the classic lists from its keys and ranks)
+    // says whether its buckets hold the lists (0), overflowed (2) or were not
+    // used (the classic lists from its counts, bin_place_kernel)
     if (w.mode && !counted && cudaMemsetAsync(w.mode, 1, sizeof(int), st) != cudaSuccess) return FPM_ERR_CUDA;
-    const bool recount = counted && w.mode != nullptr;
     const dim3 grid(grid_for(np, 256), nslot);
-#define FPM_BIN(W, L) bin_count_kernel<W, L><<<grid, 256, 0, st>>>(g, bg, w.count, w.hcount, w.hrank, w.keys, disp_ss, \
-                                                                active, recount ? w.mode : nullptr)
-    if (!counted || recount) {
+#define FPM_BIN_ALL(K)                                              \
+    do {                                                            \
+        if (cic) {                                                  \
+            if (bs == 16) K(FPM_WINDOW_CIC, 4);                     \
+            else if (bs == 8) K(FPM_WINDOW_CIC, 3);                 \
+            else K(FPM_WINDOW_CIC, 2);                              \
+        } else {                                                    \
+            if (bs == 16) K(FPM_WINDOW_TSC, 4);                     \
+            else if (bs == 8) K(FPM_WINDOW_TSC, 3);                 \
+            else K(FPM_WINDOW_TSC, 2);                              \
+        }                                                           \
+    } while (0)
+#define FPM_BIN(W, L) bin_count_kernel<W, L><<<grid, 256, 0, st>>>(g, bg, w.count, w.hcount, w.hrank, w.keys, disp_ss, active)
+    if (!counted) {
         FPM_TRACE("paint_bin_count", st);
-        if (recount) {   // both kernels return at once unless a bucket overflowed
-            bucket_overflow_reset_kernel<<<grid_for(ncounts, 256), 256, 0, st>>>(w.mode, w.count, ncounts);
-            fpm_trace::add_launches(1);
-        }
-        if (cic) {
-            if (bs == 16) FPM_BIN(FPM_WINDOW_CIC, 4);
-            else if (bs == 8) FPM_BIN(FPM_WINDOW_CIC, 3);
-            else FPM_BIN(FPM_WINDOW_CIC, 2);
-        } else {
-            if (bs == 16) FPM_BIN(FPM_WINDOW_TSC, 4);
-            else if (bs == 8) FPM_BIN(FPM_WINDOW_TSC, 3);
-            else FPM_BIN(FPM_WINDOW_TSC, 2);
-        }
+        FPM_BIN_ALL(FPM_BIN);
         if ((rc = fpm_launch_status())) return rc;
     }
 #undef FPM_BIN
     {
         FPM_TRACE("paint_bin_scan", st);
         const long long nchunk = (nbrick + 1023) / 1024;
-        if (nchunk <= 4096) {   // pass 2 sums up to nchunk partials per CTA
+        // one launch for up to two chunks; pass 2 of the two sums up to nchunk partials per CTA
+        if (nchunk > 2 && nchunk <= 4096) {
             const dim3 sgrid((unsigned)nchunk, nslot);
             brick_chunk_sum_kernel<<<sgrid, 1024, 0, st>>>(w.count, w.hcount, (int)nbrick, w.part, w.stride,
                                                            w.pstride, active);
@@ -2207,13 +2253,23 @@ int paint_sorted_impl(float* mesh, long long mesh_ss, int n, double boxsize, con
     }
     {
         FPM_TRACE("paint_bin_fill", st);
-        bin_fill_kernel<<<grid, 256, 0, st>>>(w.keys, w.hrank, np, bg, w.off, w.back, w.entries, active, w.mode);
+        if (counted && w.mode) {
+            const unsigned small = grid.x < 152 * 4 ? grid.x : 152 * 4;
+#define FPM_PLACE(W, L) bin_place_kernel<W, L><<<small, 256, 0, st>>>(g, bg, w.mode, w.off, w.hcount, w.back, w.entries)
+            FPM_BIN_ALL(FPM_PLACE);
+#undef FPM_PLACE
+        } else {
+            bin_fill_kernel<<<grid, 256, 0, st>>>(w.keys, w.hrank, np, bg, w.off, w.back, w.entries, active);
+        }
         if ((rc = fpm_launch_status())) return rc;
     }
+#undef FPM_BIN_ALL
     FPM_TRACE(cic ? "paint_cic" : "paint_tsc", st);
     const dim3 pgrid((unsigned)nbrick, nslot);
     BucketLists bl;
     bl.mode = counted ? w.mode : nullptr;
+    bl.limits = w.limits;
+    bl.hcount = w.hcount;
     bl.home = w.bucket_h;
     bl.tail = w.bucket_t;
     bl.cursor = w.cursor;
@@ -2308,9 +2364,9 @@ int fpm_kick_drift_bin(float* p, uint16_t* p_c, float* s, uint16_t* s_c, const f
     cudaStream_t st = (cudaStream_t)stream;
     if (cudaMemsetAsync(w.count, 0, (size_t)(w.hcount - w.count + w.stride) * sizeof(int), st) != cudaSuccess)
         return FPM_ERR_CUDA;
-    // option 26: the new positions straight into bucketed lists (mode word 0;
-    // an overflow sets it to 2), else the keys and ranks of the classic fill
-    // (mode word nonzero: memset bytes of 1)
+    // option 26: the new positions straight into bucketed lists (mode word 0,
+    // zeroed with the counts; an overflow sets it to 2), else counts alone are
+    // used by the paint (mode word nonzero: memset bytes of 1)
     const bool bucket = g_bucket != 0 && w.mode != nullptr;
     Buckets bk;
     bk.home = w.bucket_h;
@@ -2320,12 +2376,11 @@ int fpm_kick_drift_bin(float* p, uint16_t* p_c, float* s, uint16_t* s_c, const f
     bk.lh = g_bucket >= 2 && g_bucket < w.ch ? g_bucket : w.ch;
     bk.lt = g_bucket >= 2 && g_bucket / 2 < w.ct ? (g_bucket / 2 > 0 ? g_bucket / 2 : 1) : w.ct;
     bk.mode = w.mode;
+    bk.limits = w.limits;
     bk.spill = w.spill;
     bk.nspill = w.nspill;
     bk.spill_cap = w.spill_cap;
-    if (w.mode && (cudaMemsetAsync(w.mode, bucket ? 0 : 1, sizeof(int), st) != cudaSuccess ||
-                   cudaMemsetAsync(w.nspill, 0, sizeof(int), st) != cudaSuccess))
-        return FPM_ERR_CUDA;
+    if (w.mode && !bucket && cudaMemsetAsync(w.mode, 1, sizeof(int), st) != cudaSuccess) return FPM_ERR_CUDA;
     if (np == 0) return FPM_OK;
     const float k1 = (float)fac_k1, k2 = (float)fac_k2, d = (float)fac_d;
     FPM_TRACE("kick_drift_bin", st);
