@@ -368,7 +368,9 @@ template <int N, int TZ_ = 8, int PLAN = 0> struct Pipe {
     using PL = typename std::conditional<
         PLAN == 1, ColPlan<N>, typename std::conditional<PLAN >= 2, Plan2<N>, Plan<N>>::type>::type;
     static constexpr int TZ = TZ_;
-    static constexpr int MINB = TZ_ == 8 ? 1 : 2;
+    // n = 512: two CTAs of 256 threads fit the shared memory and cap the registers
+    // at 128 (y 239 -> 218 us, x 494 -> 374 against one CTA)
+    static constexpr int MINB = N == 512 || TZ_ != 8 ? 2 : 1;
     static constexpr int THREADS = PL::T * TZ;
     static constexpr int NZT = (N / 2 + 1 + TZ - 1) / TZ;
     static constexpr int TILE = N * TZ;  // float2 per tile
@@ -1647,7 +1649,8 @@ template <int N> int set_smem(const void* fn, int bytes) {
 template <int N, int AXIS, int DIR, bool FWD>
 int launch_col(const PassArgs& a, cudaStream_t st, int nslot = 1) {
     constexpr int TZ = ColTZ<N>::v, T = ColPlan<N>::T;
-    const int smem = (FWD ? 2 : 1) * N * TZ * (int)sizeof(float2);
+    // (with one output the spectrum stays in registers)
+    const int smem = (FWD && a.nout > 1 ? 2 : 1) * N * TZ * (int)sizeof(float2);
     auto fn = col_pass<N, AXIS, DIR, FWD>;
     int rc = set_smem<N>((const void*)fn, smem);
     if (rc) return rc;
