@@ -156,13 +156,26 @@ template <bool CG> FPM_DEV float2 ldg2(const float2* p) { return CG ? __ldcg(p) 
 // after a barrier) with a proxy fence of its own, before the barrier.
 FPM_DEV void fence_async_writes() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+// x-blocked complex mesh: [x / XB][y][x % XB][z].  The x lines of an [x][y][z] mesh of
+// n = 1024 step 4.3 MB between 64-byte pieces and copy at 3250 GB/s; in blocks of
+// XB = 8 planes they reach 5030 GB/s and the y lines (35 KB steps) lose 1 %.  So at
+// n = 1024 the y pass before the x pass writes this layout and the one after it
+// reads it (x pass 3420 -> 3116 us; blocks of 2 planes copy at 4590 GB/s, 32 at 5080; no
+// gain at n = 512, whose x lines copy as fast as its y lines).  The x pass is then
+// bound by its own instructions and barriers (radix-32 plans 3317 us).
+#define FPM_XB 8
+template <int N> FPM_DEV long long xblk_at(int x, int y, int zp) {
+    const unsigned ux = (unsigned)x;
+    return ((long long)(ux / FPM_XB * N + (unsigned)y) * FPM_XB + ux % FPM_XB) * zp;
+}
+
 // One tile: TZ consecutive l-columns (z = zt * TZ + c) of the line set oidx.
 // AXIS 1 = y lines (oidx = x plane), AXIS 0 = x lines (oidx = y row).
 // FWD: first transform in0 forward into shared memory (then the outputs are
 // inverse transforms of it); otherwise every output transforms its own input
 // in direction DIR.  blockDim.x must be Plan<N>::T * TZ.
 template <int N, int TZ, int AXIS, int DIR, bool FWD, bool CG, bool SRC_SM = false,
-          class PL = ColPlan<N>, int PADSH = 0, bool TWOA = FPM_COL_TWO_AREAS>
+          class PL = ColPlan<N>, int PADSH = 0, bool TWOA = FPM_COL_TWO_AREAS, bool OUTB = false>
 FPM_DEV void col_tile(const PassArgs& a, int zt, int o_idx, float2* smem, int slot = 0,
                       float2* tin = nullptr) {
     // SRC_SM: the input tile [N][TZ] is already in shared memory at tin (a
@@ -188,6 +201,16 @@ FPM_DEV void col_tile(const PassArgs& a, int zt, int o_idx, float2* smem, int sl
         base = (long long)o_idx * a.zp + z;
         estride = (long long)N * a.zp;
     }
+    // element pos of the line in the output (OUTB: x-blocked mesh)
+    // (an x line's outputs of one thread all sit at positions t mod XB, so they too
+    // are a constant step apart)
+    static_assert(!OUTB || PL::T % FPM_XB == 0, "a thread's positions share their place in the x blocks");
+    const long long obase = !OUTB ? base
+                            : AXIS == 1
+                                ? xblk_at<N>(o_idx, 0, a.zp) + z
+                                : (long long)o_idx * FPM_XB * a.zp + z + (long long)(t % FPM_XB) * (1 - N) * a.zp;
+    const long long ostride = OUTB && AXIS == 1 ? (long long)FPM_XB * a.zp : estride;
+    auto oat = [&](int pos) -> long long { return obase + pos * ostride; };
     auto SMW = [&](int pos) -> float2& { return work[(PADSH ? pos + (pos >> PADSH) : pos) * TZ + c]; };
     // k-vector of the transverse axes (x pass: the y index of this line, and z)
     const int ny = signed_n<N>(o_idx);
@@ -237,7 +260,7 @@ FPM_DEV void col_tile(const PassArgs& a, int zt, int o_idx, float2* smem, int sl
         }
         float2* dst = (float2*)a.out[0] + slot * a.out_ss[0];
         auto ST = [&](int pos, float2 x) {
-            if (valid) dst[base + pos * estride] = x;
+            if (valid) dst[oat(pos)] = x;
         };
         if (SRC_SM && TWOA) LI::template run2<LF::NX & 1>(u, t, SMW, SMT, ST);
         else LI::run(u, t, SMW, ST);
@@ -275,7 +298,7 @@ FPM_DEV void col_tile(const PassArgs& a, int zt, int o_idx, float2* smem, int sl
             return valid ? ldg2<CG>(src + base + pos * estride) : make_float2(0.f, 0.f);
         };
         auto ST = [&](int pos, float2 x) {
-            if (valid) dst[base + pos * estride] = x;
+            if (valid) dst[oat(pos)] = x;
         };
         LI::load(v, t, LD);
         const bool lap = AXIS == 0 && a.laplace;
@@ -383,7 +406,9 @@ template <int N, int TZ_ = 8, int PLAN = 0> struct Pipe {
 // Thread 0 loads tile `tile` (TZ l-columns x N line elements) into buf with
 // N / 256 TMA box copies of {TZ, 256} elements from the 3-D tensor map of the
 // complex mesh (dims zp, n, n; 8-byte elements), completion on bar.
-template <int N, int AXIS, int TZ>
+// INB: the mesh is x-blocked, a 4-D map (dims zp, XB, n, n / XB) whose boxes
+// also hold 256 line elements: {TZ, XB, 1, 256 / XB} for x, {TZ, 1, 256, 1} for y.
+template <int N, int AXIS, int TZ, bool INB = false>
 FPM_DEV void pipe_issue(const CUtensorMap* tm, int tile, float2* buf, uint64_t* bar) {
     using P = Pipe<N, TZ>;
     const int zt = tile % P::NZT, o_idx = tile / P::NZT;
@@ -393,6 +418,18 @@ FPM_DEV void pipe_issue(const CUtensorMap* tm, int tile, float2* buf, uint64_t* 
 #pragma unroll
     for (int j = 0; j < N / 256; ++j) {
         const int c0 = zt * P::TZ;
+        if (INB) {
+            const int c1 = AXIS == 1 ? o_idx % FPM_XB : 0;
+            const int c2 = AXIS == 1 ? j * 256 : o_idx;
+            const int c3 = AXIS == 1 ? o_idx / FPM_XB : j * (256 / FPM_XB);
+            asm volatile(
+                "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes"
+                " [%0], [%1, {%2, %3, %4, %5}], [%6];"
+                ::"r"(smem_u32(buf + j * 256 * P::TZ)), "l"(tm), "r"(c0), "r"(c1), "r"(c2), "r"(c3),
+                  "r"(smem_u32(bar))
+                : "memory");
+            continue;
+        }
         const int c1 = AXIS == 1 ? j * 256 : o_idx;
         const int c2 = AXIS == 1 ? o_idx : j * 256;
         asm volatile(
@@ -404,7 +441,7 @@ FPM_DEV void pipe_issue(const CUtensorMap* tm, int tile, float2* buf, uint64_t* 
     }
 }
 
-template <int N, int AXIS, int DIR, bool FWD, int TZ = 8, int PLAN = 0>
+template <int N, int AXIS, int DIR, bool FWD, int TZ = 8, int PLAN = 0, bool INB = false, bool OUTB = false>
 __global__ void __launch_bounds__(Pipe<N, TZ, PLAN>::THREADS, Pipe<N, TZ, PLAN>::MINB)
 col_pipe(PassArgs a, const __grid_constant__ CUtensorMap tm, int* err, int spin0) {
     // spin0 > 0 lowers the limit of each tile's first wait (option 21, to
@@ -431,12 +468,12 @@ col_pipe(PassArgs a, const __grid_constant__ CUtensorMap tm, int* err, int spin0
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    if (blockIdx.x < ntiles && threadIdx.x == 0) pipe_issue<N, AXIS, TZ>(&tm, blockIdx.x, buf(0), &bar[0]);
+    if (blockIdx.x < ntiles && threadIdx.x == 0) pipe_issue<N, AXIS, TZ, INB>(&tm, blockIdx.x, buf(0), &bar[0]);
     int it = 0;
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++it) {
         const int b = it & 1;
         const int nxt = tile + gridDim.x;
-        if (nxt < ntiles && threadIdx.x == 0) pipe_issue<N, AXIS, TZ>(&tm, nxt, buf(b ^ 1), &bar[b ^ 1]);
+        if (nxt < ntiles && threadIdx.x == 0) pipe_issue<N, AXIS, TZ, INB>(&tm, nxt, buf(b ^ 1), &bar[b ^ 1]);
         if (threadIdx.x == 0)
             sh_ok = mbar_wait_bounded(&bar[b], (uint32_t)((it >> 1) & 1), spin0 > 0 ? spin0 : FPM_MBAR_SPIN) ? 1 : 0;
         __syncthreads();
@@ -449,7 +486,7 @@ col_pipe(PassArgs a, const __grid_constant__ CUtensorMap tm, int* err, int spin0
             __syncthreads();
             return;
         }
-        col_tile<N, P::TZ, AXIS, DIR, FWD, false, true, typename P::PL, P::PADSH, P::TWOA>(
+        col_tile<N, P::TZ, AXIS, DIR, FWD, false, true, typename P::PL, P::PADSH, P::TWOA, OUTB>(
             a, tile % P::NZT, tile / P::NZT, work, 0, buf(b));
     }
 }
@@ -1726,7 +1763,7 @@ struct Options {
     int pipe1 = 0;                         // single-output column passes: two CTAs per SM, one buffer each
     int spin0 = 0;                         // > 0: spin limit of each tile's first wait in the column pipes
     // two-stage radix-32 plans in the column pipes (1, 2: y and x passes at n = 512
-    // and 1024; 3, default: the y passes at n = 1024, 1.99 against 2.03 ms)
+    // and 1024; 3, default: the y passes at n = 1024, 1.69 against 1.99 ms)
     int pipe_plan2 = 3;
 };
 thread_local Options g_opt;
@@ -1755,10 +1792,22 @@ EncodeTiledFn encode_tiled() {
 
 // tensor map of a complex half mesh (dims zp, n, n; 8-byte elements) with a
 // {TZ, 256, 1} box (y lines) or {TZ, 1, 256} box (x lines)
-template <int N, int AXIS, int TZ = 8> int pipe_map(const void* base, int zp, CUtensorMap* tm) {
+template <int N, int AXIS, int TZ = 8, bool INB = false> int pipe_map(const void* base, int zp, CUtensorMap* tm) {
     EncodeTiledFn enc = encode_tiled();
     if (enc == nullptr) return FPM_ERR_CUDA;
     if (((uintptr_t)base & 15) != 0) return FPM_ERR_ARG;
+    if (INB) {   // x-blocked mesh
+        const cuuint64_t bd[4] = {(cuuint64_t)zp, FPM_XB, (cuuint64_t)N, (cuuint64_t)(N / FPM_XB)};
+        const cuuint64_t bs[3] = {(cuuint64_t)zp * 8, (cuuint64_t)FPM_XB * zp * 8, (cuuint64_t)N * FPM_XB * zp * 8};
+        const cuuint32_t bb[4] = {(cuuint32_t)TZ, AXIS == 1 ? 1u : (cuuint32_t)FPM_XB, AXIS == 1 ? 256u : 1u,
+                                  AXIS == 1 ? 1u : 256u / FPM_XB};
+        const cuuint32_t be[4] = {1, 1, 1, 1};
+        return enc(tm, CU_TENSOR_MAP_DATA_TYPE_INT64, 4, const_cast<void*>(base), bd, bs, bb, be,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS
+                   ? FPM_OK
+                   : FPM_ERR_CUDA;
+    }
     const cuuint64_t dims[3] = {(cuuint64_t)zp, (cuuint64_t)N, (cuuint64_t)N};
     const cuuint64_t strides[2] = {(cuuint64_t)zp * 8, (cuuint64_t)N * zp * 8};
     const cuuint32_t box[3] = {(cuuint32_t)TZ, AXIS == 1 ? 256u : 1u, AXIS == 1 ? 1u : 256u};
@@ -1770,15 +1819,15 @@ template <int N, int AXIS, int TZ = 8> int pipe_map(const void* base, int zp, CU
     return FPM_OK;
 }
 
-template <int N, int AXIS, int DIR, bool FWD, int TZ = 8, int PLAN = 0>
+template <int N, int AXIS, int DIR, bool FWD, int TZ = 8, int PLAN = 0, bool INB = false, bool OUTB = false>
 int launch_pipe_tz(const PassArgs& a, int* err, cudaStream_t st) {
     using P = Pipe<N, TZ, PLAN>;
     static_assert(N % 256 == 0, "pipelined passes tile lines in boxes of 256");
-    auto fn = col_pipe<N, AXIS, DIR, FWD, TZ, PLAN>;
+    auto fn = col_pipe<N, AXIS, DIR, FWD, TZ, PLAN, INB, OUTB>;
     if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, P::SMEM) != cudaSuccess)
         return FPM_ERR_CUDA;
     CUtensorMap tm;
-    int rc = pipe_map<N, AXIS, TZ>(a.in[0], a.zp, &tm);
+    int rc = pipe_map<N, AXIS, TZ, INB>(a.in[0], a.zp, &tm);
     if (rc) return rc;
     static const char* names[2][2][2] = {{{"fft_x_fwd", "fft_x_fwd"}, {"fft_x_inv", "fft_x_fwd_transfer_inv"}},
                                          {{"fft_y_fwd", "fft_y_fwd"}, {"fft_y_inv", "fft_y_inv"}}};
@@ -1815,7 +1864,7 @@ int launch_pipe(const PassArgs& a, int* err, cudaStream_t st) {
         if (g_opt.pipe_plan2 == 1) return launch_pipe_tz<N, AXIS, DIR, FWD, 8, 2>(a, err, st);
         if (g_opt.pipe_plan2 == 2) return launch_pipe_tz<N, AXIS, DIR, FWD, 8, 3>(a, err, st);
         if constexpr (AXIS == 1 && N == 1024) {
-            if (g_opt.pipe_plan2 == 3) return launch_pipe_tz<N, AXIS, DIR, FWD, 8, 2>(a, err, st);
+            if (g_opt.pipe_plan2 == 3) return launch_pipe_tz<N, AXIS, DIR, FWD, 8, 3>(a, err, st);
         }
     }
     return launch_pipe_tz<N, AXIS, DIR, FWD, 8>(a, err, st);
@@ -2079,6 +2128,9 @@ template <int N> struct Pipelines {
         PassArgs a = base_args(N, boxsize);
         a.in[0] = b0;
         add_out(a, 0, 0, 1.f, b0);
+        // the y and x passes through the x-blocked layout (n = 1024, one potential)
+        const bool xb = N == 1024 && (g_opt.stencil || packed || phi_out) && g_opt.pipe && !g_opt.pipe1 &&
+                        !g_opt.pipe_xcol && g_opt.pipe_plan2 == 3 && !g_opt.fused[0][N < 1024];
         bool done = false;
         if constexpr (N >= 512) {
             if (q != nullptr && g_opt.fused[0][N < 1024]) {
@@ -2098,7 +2150,14 @@ template <int N> struct Pipelines {
                 }
             }
             if (!piped && (rc = launch_r2c<N>(rho, b0, complex_row(N), 1.f, st))) return rc;
-            if ((rc = col_any<N, 1, -1, false>(a, q ? &q->error : nullptr, st))) return rc;
+            if (xb) {
+                if constexpr (N == 1024) {
+                    a.out[0] = b1;
+                    if ((rc = launch_pipe_tz<N, 1, -1, false, 8, 3, false, true>(a, &q->error, st))) return rc;
+                }
+            } else if ((rc = col_any<N, 1, -1, false>(a, q ? &q->error : nullptr, st))) {
+                return rc;
+            }
         }
         if (g_opt.stencil || packed || phi_out) {
             // potential only: x forward + laplace + x inverse (one output), y
@@ -2113,11 +2172,20 @@ template <int N> struct Pipelines {
             x.shell = shell;
             add_out(x, 0, 0, 1.f, b0);
             int* err = q ? &q->error : nullptr;
-            if ((rc = col_any<N, 0, +1, true>(x, err, st))) return rc;
             PassArgs y = base_args(N, boxsize);
             y.in[0] = b0;
             add_out(y, 0, 0, 1.f, b0);
-            if ((rc = col_any<N, 1, +1, false>(y, err, st))) return rc;
+            if (xb) {
+                if constexpr (N == 1024) {
+                    x.in[0] = y.in[0] = b1;
+                    x.out[0] = b1;
+                    if ((rc = launch_pipe_tz<N, 0, +1, true, 8, 0, true, true>(x, err, st))) return rc;
+                    if ((rc = launch_pipe_tz<N, 1, +1, false, 8, 3, true, false>(y, err, st))) return rc;
+                }
+            } else {
+                if ((rc = col_any<N, 0, +1, true>(x, err, st))) return rc;
+                if ((rc = col_any<N, 1, +1, false>(y, err, st))) return rc;
+            }
             float* phi = (float*)b1;   // a complex buffer holds a real mesh
             PassArgs z = base_args(N, boxsize);
             z.in[0] = b0;

@@ -104,11 +104,12 @@ int fpm_device_init(void);
  *     the two-stage plan with a radix-32 first stage (one shared-memory
  *     exchange per 1024-point transform), its single-output tiles exchanging
  *     in two areas (1) or in the padded work area alone (2); 3 (default): the
- *     two-stage plan for the y passes at n = 1024 only (1.99 against 2.03 ms
- *     per pass; the x pass measured slower with it, 3.60 against 3.46 ms).
+ *     latter for the y passes at n = 1024 only (1.69 against 1.99 ms per pass;
+ *     the x pass measured slower with it, 3.32 against 3.12 ms), and at that
+ *     size the x pass of the potential works on an x-blocked mesh.
  * 26: brick lists of fpm_kick_drift_bin + fpm_paint_sorted_counted through
- *     per-brick buckets (1, default: no fill pass), or from brick keys and
- *     home ranks filled by a pass of their own (0); k >= 2: buckets holding at
+ *     per-brick buckets (1, default: no fill pass), or with counts alone and
+ *     the ids placed by a pass of their own (0); k >= 2: buckets holding at
  *     most k home and k / 2 tail entries (forces the overflow path; testing).
  * 25: warp-aggregated brick deposit (1) for 16^3-cell bricks with 19-word
  *     rows: lanes of a warp whose windows start in the same cell sum each
@@ -158,7 +159,7 @@ int fpm_paint_sorted_add(float* mesh, int n, double boxsize, const float* disp, 
  * paint's.  With option 26 (default on) the pass stores each particle id
  * straight into its bricks' buckets in the workspace, and the counted paint
  * copies them into its particle lists while it deposits (no fill pass); a
- * bucket that would overflow makes that paint recount and fill instead.
+ * spill list that would overflow makes that paint place the ids itself.
  * Either way the lists the readouts read are the same.  Replaces
  * core.py:168-180 (K, K, D) + the first half of the mass assignment of
  * core.py:191.                                                             */
