@@ -340,6 +340,45 @@ col_pass(PassArgs a) {
     col_tile<N, ColTZ<N>::v, AXIS, DIR, FWD, false>(a, blockIdx.x, blockIdx.y, smem, slot);
 }
 
+// One output, no transfer (r2c, c2r and the y passes of a force): without the
+// transfer's code the lines fit fewer registers, so n = 1024 and the y lines of
+// n = 512 take the radix-16 plan (two exchanges, 16 loads in flight per thread) at
+// 64 registers: n = 1024 y 2654 -> 1873 us, x 3020 -> 2812; n = 512 y 260 -> 202 (the
+// pipelined pass 217), x 300 -> 292 (radix-8 plan; 310 with radix 16); n = 384 121
+// -> 106, 192 17 -> 15.
+template <int N, int AXIS> struct PlainPlan {
+    static constexpr bool row = N == 1024 || (N == 512 && AXIS == 1);
+    using PL = typename std::conditional<row, Plan<N>, ColPlan<N>>::type;
+    static constexpr int TZ = ColTZ<N>::v;
+    static constexpr int MINB = N == 1024 ? 2 : N == 512 ? (row ? 4 : 2) : ColMinB<N>::v;
+};
+template <int N, int AXIS, int DIR>
+__global__ void __launch_bounds__(PlainPlan<N, AXIS>::PL::T * PlainPlan<N, AXIS>::TZ, PlainPlan<N, AXIS>::MINB)
+col_plain(PassArgs a) {
+    using P = PlainPlan<N, AXIS>;
+    using PL = typename P::PL;
+    using LI = LineFFT<N, PL::T, DIR, typename PL::R, false>;
+    constexpr int TZ = P::TZ;
+    extern __shared__ float2 smem[];
+    const int slot = blockIdx.z;
+    if (a.slot_active && !a.slot_active[slot]) return;
+    const int c = threadIdx.x % TZ, t = threadIdx.x / TZ;
+    const int z = blockIdx.x * TZ + c;
+    const bool valid = z < N / 2 + 1;
+    const long long estride = AXIS == 1 ? a.zp : (long long)N * a.zp;
+    const long long base = (AXIS == 1 ? (long long)blockIdx.y * N * a.zp : (long long)blockIdx.y * a.zp) + z;
+    const float2* src = a.in[0] + slot * a.in_ss[0] + base;
+    float2* dst = (float2*)a.out[0] + slot * a.out_ss[0] + base;
+    auto SM = [&](int pos) -> float2& { return smem[pos * TZ + c]; };
+    auto LD = [&](int pos) -> float2 { return valid ? src[pos * estride] : make_float2(0.f, 0.f); };
+    auto ST = [&](int pos, float2 x) {
+        if (valid) dst[pos * estride] = x;
+    };
+    float2 v[PL::E];
+    LI::load(v, t, LD);
+    LI::run(v, t, SM, ST);
+}
+
 // ---------------------------------------------------------------------------
 // Pipelined y / x pass (persistent, one CTA per SM, single input).  Warp 0
 // streams tile i+1 into one shared-memory buffer with cp.async.bulk row-
@@ -1686,15 +1725,25 @@ template <int N> int set_smem(const void* fn, int bytes) {
 template <int N, int AXIS, int DIR, bool FWD>
 int launch_col(const PassArgs& a, cudaStream_t st, int nslot = 1) {
     constexpr int TZ = ColTZ<N>::v, T = ColPlan<N>::T;
+    // [AXIS][inverse][FWD]: the FWD variant (forward then inverse outputs) only exists for x
+    static const char* names[2][2][2] = {{{"fft_x_fwd", "fft_x_fwd"}, {"fft_x_inv", "fft_x_fwd_transfer_inv"}},
+                                         {{"fft_y_fwd", "fft_y_fwd"}, {"fft_y_inv", "fft_y_inv"}}};
+    if (!FWD && a.nout == 1 && a.o[0].src == 0 && a.o[0].pw == 0 && a.o[0].coef == 1.f && !a.laplace) {
+        using P = PlainPlan<N, AXIS>;
+        const int smem1 = N * P::TZ * (int)sizeof(float2);
+        auto fn1 = col_plain<N, AXIS, DIR>;
+        int rc = set_smem<N>((const void*)fn1, smem1);
+        if (rc) return rc;
+        FPM_TRACE(names[AXIS][DIR > 0][0], st);
+        fn1<<<dim3((N / 2 + 1 + P::TZ - 1) / P::TZ, N, nslot), P::PL::T * P::TZ, smem1, st>>>(a);
+        return fpm_launch_status();
+    }
     // (with one output the spectrum stays in registers)
     const int smem = (FWD && a.nout > 1 ? 2 : 1) * N * TZ * (int)sizeof(float2);
     auto fn = col_pass<N, AXIS, DIR, FWD>;
     int rc = set_smem<N>((const void*)fn, smem);
     if (rc) return rc;
     dim3 grid((N / 2 + 1 + TZ - 1) / TZ, N, nslot);
-    // [AXIS][inverse][FWD]: the FWD variant (forward then inverse outputs) only exists for x
-    static const char* names[2][2][2] = {{{"fft_x_fwd", "fft_x_fwd"}, {"fft_x_inv", "fft_x_fwd_transfer_inv"}},
-                                         {{"fft_y_fwd", "fft_y_fwd"}, {"fft_y_inv", "fft_y_inv"}}};
     FPM_TRACE(names[AXIS][DIR > 0][FWD ? 1 : 0], st);
     fn<<<grid, T * TZ, smem, st>>>(a);
     return fpm_launch_status();
@@ -1978,7 +2027,9 @@ template <int N> int launch_stencil(const float* phi, float* fx, float* fy, floa
 template <int N, int AXIS, int DIR, bool FWD>
 int col_any(const PassArgs& a, int* err, cudaStream_t st) {
     if constexpr (N >= 512) {
-        if (err != nullptr && g_opt.pipe) return launch_pipe<N, AXIS, DIR, FWD>(a, err, st);
+        // (the y lines of n = 512 run faster unpipelined: see PlainPlan)
+        const bool plain = N == 512 && AXIS == 1 && g_opt.pipe_plan2 == 3 && !g_opt.pipe1;
+        if (err != nullptr && g_opt.pipe && !plain) return launch_pipe<N, AXIS, DIR, FWD>(a, err, st);
     }
     return launch_col<N, AXIS, DIR, FWD>(a, st);
 }
