@@ -1446,14 +1446,15 @@ row_c2r_lpt2(PassArgs a) {
             if (o == 0) {
                 sum[slot] = x;
             } else if (o == 1) {
-                acc[slot] = make_float2(sum[slot].x * x.x, sum[slot].y * x.y);
+                // (rounded here: the next output's product is the one to contract)
+                acc[slot] = make_float2(__fmul_rn(sum[slot].x, x.x), __fmul_rn(sum[slot].y, x.y));
                 sum[slot] = c_add(sum[slot], x);
             } else if (o == 2) {
-                acc[slot].x += x.x * sum[slot].x;
-                acc[slot].y += x.y * sum[slot].y;
+                acc[slot].x = __fmaf_rn(x.x, sum[slot].x, acc[slot].x);
+                acc[slot].y = __fmaf_rn(x.y, sum[slot].y, acc[slot].y);
             } else {
-                acc[slot].x -= x.x * x.x;
-                acc[slot].y -= x.y * x.y;
+                acc[slot].x = __fmaf_rn(-x.x, x.x, acc[slot].x);
+                acc[slot].y = __fmaf_rn(-x.y, x.y, acc[slot].y);
                 if (o == 5) out[pos] = c_scale(acc[slot], sc);
             }
             ++slot;
@@ -1484,9 +1485,10 @@ FPM_DEV void philox4x32_10(uint32_t c[4], uint32_t k0, uint32_t k1) {
 }
 // Mode values.  The reference numbers are float64 (Box-Muller of two 53-bit
 // uniforms), rounded to float32; in FP64 the logarithm, square root and
-// sincospi bound the kernel (256^3: 1550 us).  Here they are float-float
-// (ff.cuh), good to about 2^-38, so all but some 1e-4 of the modes round to
-// the same float32 and the error against float64 is the rounding either way.
+// sincospi bound the kernel.  Here they are float-float
+// (ff.cuh), good to about 2^-42, so all but some 1e-6 of the modes round to
+// the same float32 and the error against float64 is the rounding either way
+// (256^3: 1551 -> 141 us).
 //   log: table-driven (Tang 1990), u = 2^e f with f inv_k = 1 + r, |r| <= 2^-7,
 //     and the series of log(1 + r); entries next to f = 1 and 2 have inv_k = 1
 //     and 1/2 exactly, so r keeps the relative accuracy of -log(u) at u -> 1.
@@ -1555,14 +1557,17 @@ FPM_DEV void wn_sincos(unsigned long long V, ff& c, ff& s) {
     const float a = dh * 0x1p-54f;
     ff th = ff_two_prod(a, TPH);
     th = ff_quick(th.h, __fmaf_rn(a, TPL, __fmaf_rn(dl * 0x1p-54f, TPH, th.l)));
-    const float x = th.h, x2 = x * x;
-    const float ds = x * x2 * __fmaf_rn(x2, 1.f / 120.f, -1.f / 6.f);       // sin - theta
-    const float c1 = x2 * __fmaf_rn(x2, __fmaf_rn(x2, -1.f / 720.f, 1.f / 24.f), -0.5f);   // cos - 1
+    const float x = th.h;
+    ff x2 = ff_two_prod(x, x);                                              // theta^2
+    x2 = ff_quick(x2.h, __fmaf_rn(2.f * x, th.l, x2.l));
+    const float ds = x * x2.h * __fmaf_rn(x2.h, 1.f / 120.f, -1.f / 6.f);   // sin - theta
     const ff sn = ff_quick(th.h, __fadd_rn(th.l, ds));
+    // cos - 1 = -theta^2 / 2 + theta^4 / 24 - theta^6 / 720
+    const ff c1 = ff_quick(-0.5f * x2.h, __fmaf_rn(x2.h * x2.h, __fmaf_rn(x2.h, -1.f / 720.f, 1.f / 24.f), -0.5f * x2.l));
     // cos(A + th) = C + (C c1 - S sin th), sin(A + th) = S + (S c1 + C sin th)
-    const ff cs = ff_mul(ff_of(t.z, t.w), ff_neg(sn)), cc = ff_mul(ff_of(t.x, t.y), sn);
-    c = ff_add(ff_of(t.x, t.y), ff_add_f(cs, t.x * c1));
-    s = ff_add(ff_of(t.z, t.w), ff_add_f(cc, t.z * c1));
+    const ff C = ff_of(t.x, t.y), S = ff_of(t.z, t.w);
+    c = ff_add(C, ff_add(ff_mul(C, c1), ff_neg(ff_mul(S, sn))));
+    s = ff_add(S, ff_add(ff_mul(S, c1), ff_mul(C, sn)));
 }
 FPM_DEV float ff_round_mul(ff a, ff b) {
     const ff p = ff_mul(a, b);
