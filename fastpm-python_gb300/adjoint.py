@@ -122,7 +122,9 @@ class ForwardModel(object):
         for act, f in zip(acts, fac):
             t = act[0]
             if record:
-                rec.append({k: state[k].clone() for k in ('S', 'P', 'F')})
+                # what the action's transpose reads: F for a kick, P for a drift, S for a force
+                k = {'K': 'F', 'D': 'P', 'F': 'S'}[t]
+                rec.append({k: state[k].clone()})
             if t == 'K':
                 _lib.call('fpm_kick', _lib.ptr(state['P']), _lib.ptr(state['Pc']), _lib.ptr(state['F']),
                           state['P'].numel(), f, _lib.stream_ptr())
@@ -182,10 +184,13 @@ class ForwardModel(object):
         return float((self.resid.double() ** 2).sum())
 
     # -- reverse ------------------------------------------------------------------
-    def _dot(self, x, y):
-        return float((x.double() * y.double()).sum())
+    @staticmethod
+    def _dot(x, y, out):
+        """out (one element of a zeroed float64 device array) += sum x y, in float64;
+        read back once, at the end of the reverse pass."""
+        _lib.call('fpm_dot', _lib.ptr(x), _lib.ptr(y), x.numel(), _lib.ptr(out), _lib.stream_ptr())
 
-    def _vjp_force(self, S, lamF, meshes, Fout, lamS):
+    def _vjp_force(self, S, lamF, meshes, Fout, lamS, dot):
         pm, n = self.fpm, self.n
         win = self.res
         # term 1: the window moves with the particle
@@ -211,7 +216,7 @@ class ForwardModel(object):
         _lib.call('fpm_readout_vjp', m1, 1, n, pm.L, _lib.ptr(S), None, self.np, self.nc, 0.0,
                   _lib.FPM_WINDOW[win], None, None, (ctypes.c_float * 1)(factor / self.nbar),
                   _lib.ptr(lamS), 1, _lib.stream_ptr())
-        return self._dot(lamF, Fout) / factor
+        self._dot(lamF, Fout, dot)
 
     def _lpt1_T(self, lam):
         """g = -sum_d K_d FFT(paint_Q(lam[:, d])) on the base mesh (lpt1 transpose)."""
@@ -253,28 +258,31 @@ class ForwardModel(object):
         _lib.call('fpm_readout_vjp', m1, 1, n, fpm.L, _lib.ptr(self.S_final), None, self.np, self.nc,
                   0.0, _lib.FPM_WINDOW['cic'], None, None, (ctypes.c_float * 1)(1.0), _lib.ptr(lamS), 1,
                   _lib.stream_ptr())
-        dfac = numpy.zeros(len(self.acts))       # dL/d(factor of action)
+        # device sums: per action, then the LPT coefficients, read once below
+        nact = len(self.acts)
+        dots = torch.zeros(nact + 4, dtype=torch.float64, device=dev)
         for si in reversed(range(len(self.segments))):
             a, b = self.segments[si]
             state = {k: v.clone() for k, v in self.ckpt[si].items()}
             rec = self._run(state, self.acts[a:b], self.fac[a:b], record=True)
             for j in reversed(range(b - a)):
                 act, f, r = self.acts[a + j], self.fac[a + j], rec[j]
+                dot = dots[a + j: a + j + 1]
                 if act[0] == 'K':
-                    dfac[a + j] = self._dot(lamP, r['F'])
-                    lamF += f * lamP
+                    self._dot(lamP, r['F'], dot)
+                    lamF.add_(lamP, alpha=f)
                 elif act[0] == 'D':
-                    dfac[a + j] = self._dot(lamS, r['P'])
-                    lamP += f * lamS
+                    self._dot(lamS, r['P'], dot)
+                    lamP.add_(lamS, alpha=f)
                 else:
-                    dfac[a + j] = self._vjp_force(r['S'], lamF, r['meshes'], r['Fout'], lamS)
+                    self._vjp_force(r['S'], lamF, r['meshes'], r['Fout'], lamS, dot)
                     lamF.zero_()
         D1, D2, A1, A2 = self.coefs
         # LPT
         lam1 = D1 * lamS + A1 * lamP
         lam2 = D2 * lamS + A2 * lamP
-        dco = numpy.array([self._dot(lamS, self.psi1), self._dot(lamS, self.psi2),
-                           self._dot(lamP, self.psi1), self._dot(lamP, self.psi2)])
+        for i, (lam, psi) in enumerate(((lamS, self.psi1), (lamS, self.psi2), (lamP, self.psi1), (lamP, self.psi2))):
+            self._dot(lam, psi, dots[nact + i: nact + i + 1])
         g_d = self._lpt1_T(lam1)
         g_s = self._lpt1_T(lam2)
         lam_s = g_s.c2r()
@@ -318,6 +326,9 @@ class ForwardModel(object):
         wmode = self.mode_weights(pm)
         q = self._shell_index(pm)
         gT = (wmode * (gd.conj() * self.wn.value).real.double() * dTt.double()[q]).sum()
+        sums = dots.cpu().numpy()
+        dfac, dco = sums[:nact], sums[nact:]     # dL/d(factor of action), dL/d(D1, D2, A1, A2)
+        dfac[[i for i, act in enumerate(self.acts) if act[0] == 'F']] /= 1.5 * Om
         dL_dOm = float((dfac * dfac_dOm).sum() + (dco * dco_dOm).sum() + float(gT))
         return g_wn, dL_dOm
 

@@ -380,7 +380,9 @@ int fpm_dot(const float* x, const float* y, long long n, double* out, void* stre
     if (n == 0) return FPM_OK;
     cudaStream_t st = (cudaStream_t)stream;
     FPM_TRACE("dot", st);
-    dot_kernel<<<grid_for(n, 256), 256, 0, st>>>(x, y, n, out);
+    // (few CTAs: the FP64 reduction of a CTA costs as much as some ten elements per thread)
+    const unsigned grid = grid_for(n, 256);
+    dot_kernel<<<grid < 152 * 4 ? grid : 152 * 4, 256, 0, st>>>(x, y, n, out);
     return fpm_launch_status();
 }
 
