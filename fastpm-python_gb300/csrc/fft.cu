@@ -380,7 +380,7 @@ col_plain(PassArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// Pipelined y / x pass (persistent, one CTA per SM, single input).  Warp 0
+// Pipelined y / x pass (persistent, one CTA per SM, two at n = 512; single input).  Warp 0
 // streams tile i+1 into one shared-memory buffer with cp.async.bulk row-
 // segment copies (TZ * 8 bytes each, completion counted on an mbarrier)
 // while every warp transforms tile i from the other buffer, so HBM reads are
@@ -416,9 +416,9 @@ FPM_DEV bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, int limit = FPM_M
 }
 
 // The pipelined kernels hide load latency with TMA, so they run one CTA per
-// SM and use the radix-16 plans (two shared-memory exchanges per 1024-point
-// line instead of three).
-// TZ = 8: one CTA per SM (64-byte row segments); TZ = 4 (two CTAs per SM, half
+// SM (two at n = 512) and use the radix-16 plans (two shared-memory exchanges
+// per 1024-point line instead of three).
+// TZ = 8: 64-byte row segments; TZ = 4 (two CTAs per SM, half
 // the tile, 32-byte row segments) measured 1.8x slower for the x pass at n = 1024.
 // MINB = CTAs per SM the launch bounds ask for.
 template <int N, int TZ_ = 8, int PLAN = 0> struct Pipe {
